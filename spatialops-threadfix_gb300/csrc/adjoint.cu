@@ -145,22 +145,6 @@ __global__ void __launch_bounds__(BX* BY, 4) heat_adjoint_kernel(const S* __rest
   }
 }
 
-// Face coefficients lf_d[c] = lambda[c - s_d] + lambda[c] for the faces the reverse step reads:
-// along axis d indices 0..n_d (the last one is the high face of the last cell), the other two
-// axes 0..n-1.
-__global__ void face_coef_kernel(const double* __restrict__ L, double* __restrict__ lfx, double* __restrict__ lfy,
-                                 double* __restrict__ lfz, int sy, long sz, int nx, int ny, int nz) {
-  const long total = (long)(nx + 1) * (ny + 1) * (nz + 1);
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % (nx + 1)), y = (int)((i / (nx + 1)) % (ny + 1)), z = (int)(i / ((long)(nx + 1) * (ny + 1)));
-    const long c = (long)x + (long)sy * y + sz * z;
-    const double lc = L[c];
-    if (y < ny && z < nz) lfx[c] = L[c - 1] + lc;
-    if (x < nx && z < nz) lfy[c] = L[c - sy] + lc;
-    if (x < nx && y < ny) lfz[c] = L[c - sz] + lc;
-  }
-}
-
 // dst = src rounded to FP32 (whole windows of the same layout).
 __global__ void to_f32_kernel(const double* __restrict__ src, float* __restrict__ dst, long n) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
@@ -300,11 +284,7 @@ int gradient_impl(S* spool, size_t stride, double* dpool, size_t cells, int nck,
   const View<double> vl = make_view<double>(lamf);
   const long origin = vl.base - (const double*)lamf.data;  // interior origin within a window
   double* lf[3] = {dbuf(2) + origin, dbuf(3) + origin, dbuf(4) + origin};
-  {
-    LaunchScope ls("face_coef", s);
-    face_coef_kernel<<<num_sms() * 4, 256, 0, s>>>(vl.base, lf[0], lf[1], lf[2], vl.sy, vl.sz, n[0], n[1], n[2]);
-    NEBO_LAUNCH_CHECK("nebo_heat_gradient (face coefficients)");
-  }
+  if ((rc = heat_face_coef(&lamf, lf, false, s))) return rc;
   // the forward sweep's lambda and T_0 in the state type
   nebo_field lamS = lamf;
   if constexpr (!f64) {
@@ -316,6 +296,11 @@ int gradient_impl(S* spool, size_t stride, double* dpool, size_t cells, int nck,
   } else {
     NEBO_CUDA_TRY(cudaMemcpyAsync(sbuf(0), T0->data, bytes, cudaMemcpyDeviceToDevice, s));
   }
+  // FP64 steps share the reverse sweep's face coefficients
+  const bool faces = f64 && heat_faces_ok(T0);
+  auto forward_step = [&](const nebo_field* a, const nebo_field* b) {
+    return faces ? heat_step_faces(a, b, lf, dt, unit, s) : heat_step_dispatch(a, b, &lamS, dt, unit, s);
+  };
   // forward sweep: checkpoints every L steps; the last segment's states go straight to the
   // segment buffers (they need no recomputation)
   const int klast = (nck - 1) * L;
@@ -336,7 +321,7 @@ int gradient_impl(S* spool, size_t stride, double* dpool, size_t cells, int nck,
     else
       nxt = cur == tmp0 ? tmp1 : tmp0;
     nebo_field a = state_at(cur), b = state_at(nxt);
-    rc = heat_step_dispatch(&a, &b, &lamS, dt, unit, s);
+    rc = forward_step(&a, &b);
     cur = nxt;
   }
   if (rc) return rc;
@@ -361,7 +346,7 @@ int gradient_impl(S* spool, size_t stride, double* dpool, size_t cells, int nck,
     for (int k = k0; seg != nck - 1 && k + 1 < k1 && !rc; ++k) {
       nebo_field a = state_at(k == k0 ? sbuf(seg) : sbuf(nck + (k - k0 - 1)));
       nebo_field b = state_at(sbuf(nck + (k - k0)));
-      rc = heat_step_dispatch(&a, &b, &lamS, dt, unit, s);
+      rc = forward_step(&a, &b);
     }
     for (int k = k1 - 1; k >= k0 && !rc; --k) {
       nebo_field tk = state_at(k == k0 ? sbuf(seg) : sbuf(nck + (k - k0 - 1)));

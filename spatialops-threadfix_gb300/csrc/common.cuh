@@ -93,6 +93,12 @@ void pool_retain();
 // Periodic ghost fill of one uniform-ghost patch (ghost.cu).
 int fill_periodic_any(const nebo_field* f, cudaStream_t s);
 
+// The exact FP64 heat step on face coefficients computed once per lambda (heat.cu).
+int heat_face_coef(const nebo_field* lam, double* const lf[3], bool half, cudaStream_t s);
+int heat_step_faces(const nebo_field* T, const nebo_field* To, const double* const lf[3], double dt,
+                    const double sp[3], cudaStream_t s);
+bool heat_faces_ok(const nebo_field* f);
+
 // SM count of the current device, queried once (callers on several threads may race to the
 // first query; they store the same value).
 inline int num_sms() {
