@@ -1072,6 +1072,142 @@ __global__ void __launch_bounds__(BP_THREADS, 3) heat_step_f32_bulk2_kernel(cons
   if (!ok) atomicAdd(&g_bulk_timeouts, 1u);
 }
 
+// FP32 step on slabs of full rows at any row pitch and alignment (nx <= SL_MAXX).  A block owns
+// SL_R rows, a thread one column of them.  The block's rows and the one on either side are one run
+// of a plane in memory, so one cp.async.bulk per plane and field brings them into a ring of SL_NS
+// stages, whatever the pitch: the copy starts at the 16-byte boundary below the run and ends at the
+// one above it (at most 3 floats more on either side; past the field's end it stops below instead,
+// which drops cells of plane nz's ghost corner that no face reads), and the cells are read
+// (address mod 16) bytes into the stage.  Planes below 0 are not staged (the low z faces of a
+// chunk's first plane read them from global memory), so no copy starts before the field.
+// What bounds it: issue (82 instructions per cell, 59 % of the slots) and the barrier per plane;
+// 40 registers let four blocks of 352 threads share an SM (64 registers, two blocks: 42.4 us).
+// At 323 x 197 x 150: 36.9 us = 3.1 TB/s, where 4-byte cp.async copies per cell took 108 us;
+// 322 x 198 x 150 (8-byte copies before) 69.8 -> 36.9, 401 x 301 x 201 141 -> 82.
+constexpr int SL_R = 4;        // rows per block
+constexpr int SL_NS = 3;       // stages
+constexpr int SL_MAXX = 1024;  // threads per block
+
+__host__ __device__ __forceinline__ uint32_t slab_stage_bytes(int gx) {  // bytes per field and stage
+  return ((uint32_t)((SL_R + 2) * gx + 3) * 4u + 15u) & ~15u;
+}
+
+__global__ void __maxnreg__(40)
+    heat_step_f32_slab_kernel(const float* __restrict__ tdata, float* __restrict__ tout,
+                              const float* __restrict__ ldata, long total, int gx, long sz, int nx, int ny, int nz,
+                              int zchunk, float w0, float w1, float w2) {
+  constexpr int NS = SL_NS, SR = SL_R;
+  extern __shared__ __align__(128) unsigned char slab_smem[];
+  const uint32_t fb = slab_stage_bytes(gx);
+  const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(slab_smem);
+  const uint32_t bar0 = s0 + (uint32_t)NS * 2u * fb;
+  const int x = threadIdx.x, y0 = blockIdx.x * SR;
+  const int z0 = blockIdx.y * zchunk, z1 = min(z0 + zchunk, nz);
+  if (x == 0) {
+    for (int st = 0; st < NS; ++st) mbar_init(bar0 + 8 * st, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  const int nr = min(SR, ny - y0);        // rows of the block
+  const long first = sz + (long)gx * y0;  // window element of row y0 - 1 of plane 0
+  // plane p (0 <= p <= z1) into stage st
+  auto issue = [&](int p, int st) {
+    if (p > z1) return;
+    const uint32_t bar = bar0 + 8 * st, d = s0 + (uint32_t)st * 2u * fb;
+    const long s = first + sz * p, e = s + (long)(nr + 2) * gx;
+    const uintptr_t ta = (uintptr_t)(tdata + s) & ~(uintptr_t)15, la = (uintptr_t)(ldata + s) & ~(uintptr_t)15;
+    uintptr_t te = ((uintptr_t)(tdata + e) + 15) & ~(uintptr_t)15, le = ((uintptr_t)(ldata + e) + 15) & ~(uintptr_t)15;
+    if (te > (uintptr_t)(tdata + total)) te -= 16;
+    if (le > (uintptr_t)(ldata + total)) le -= 16;
+    mbar_expect_tx(bar, (uint32_t)(te - ta) + (uint32_t)(le - la));
+    bulk_g2s(d, (const void*)ta, (uint32_t)(te - ta), bar);
+    bulk_g2s(d + fb, (const void*)la, (uint32_t)(le - la), bar);
+  };
+  if (x == 0)
+    for (int q = 0; q < NS - 1; ++q) issue(z0 + q, q);
+  const bool active = x < nx;
+  const int xc = min(x, nx - 1);
+  const bool xe = x == 0 || x == nx - 1 || y0 == 0 || y0 + SR >= ny;
+  // the shared address of the column left of the cell in the row below the block, plane p: the
+  // slab starts (address mod 16) bytes into its stage
+  const uint32_t aT = (uint32_t)((uintptr_t)tdata + 4 * first), aL = (uint32_t)((uintptr_t)ldata + 4 * first);
+  const uint32_t sz4 = (uint32_t)sz * 4u, g4 = (uint32_t)gx * 4u;
+  auto lds = [](uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+  };
+  auto offT = [&](int p, uint32_t stage) { return stage + ((aT + sz4 * (uint32_t)p) & 15u) + 4u * (uint32_t)xc; };
+  auto offL = [&](int p, uint32_t stage) { return stage + fb + ((aL + sz4 * (uint32_t)p) & 15u) + 4u * (uint32_t)xc; };
+  bool ok = mbar_wait(bar0, 0);
+  float t[SR], l[SR], fz[SR];
+  uint32_t T0 = offT(z0, s0), L0 = offL(z0, s0);
+#pragma unroll
+  for (int k = 0; k < SR; ++k) {
+    const long m = first + sz * (z0 - 1) + xc + 1 + (long)gx * min(k + 1, nr + 1);
+    t[k] = lds(T0 + (k + 1) * g4 + 4);
+    l[k] = lds(L0 + (k + 1) * g4 + 4);
+    fz[k] = (__ldg(ldata + m) + l[k]) * (t[k] - __ldg(tdata + m));
+  }
+  float* out = tout + (long)x + (long)gx * y0 + sz * z0;
+  int st = 0, ph = 0;  // stage of plane z, phase parity of plane z + 1's stage
+#pragma unroll 1
+  for (int z = z0; z < z1; ++z) {
+    const int sn = st + 1 == NS ? 0 : st + 1;
+    if (sn == 0) ph ^= 1;
+    __syncthreads();  // plane z - 1's stage is no longer read
+    if (x == 0) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      issue(z + NS - 1, st == 0 ? NS - 1 : st - 1);
+    }
+    ok &= mbar_wait(bar0 + 8 * sn, ph);
+    const uint32_t sn0 = s0 + (uint32_t)sn * 2u * fb;
+    uint32_t T1 = offT(z + 1, sn0), L1 = offL(z + 1, sn0);
+    const uint32_t Tn = T1, Ln = L1;
+    float fy = (lds(L0 + 4) + l[0]) * (t[0] - lds(T0 + 4));
+    float v[SR];
+#pragma unroll
+    for (int k = 0; k < SR; ++k) {
+      T0 += g4;
+      L0 += g4;
+      T1 += g4;
+      L1 += g4;
+      const float tc = t[k], lc = l[k];
+      const float fxl = (lds(L0) + lc) * (tc - lds(T0));
+      const float fxh = (lc + lds(L0 + 8)) * (lds(T0 + 8) - tc);
+      const float tu = k + 1 < SR ? t[k + 1 < SR ? k + 1 : k] : lds(T0 + g4 + 4);
+      const float lu = k + 1 < SR ? l[k + 1 < SR ? k + 1 : k] : lds(L0 + g4 + 4);
+      const float fyh = (lc + lu) * (tu - tc);
+      const float tn = lds(T1 + 4), ln = lds(L1 + 4);
+      const float fzh = (lc + ln) * (tn - tc);
+      v[k] = fmaf(w2, fzh - fz[k], fmaf(w1, fyh - fy, fmaf(w0, fxh - fxl, tc)));
+      fy = fyh;
+      fz[k] = fzh;
+      t[k] = tn;
+      l[k] = ln;
+    }
+    T0 = Tn;
+    L0 = Ln;
+    if (active) {
+      float* o = out;
+#pragma unroll
+      for (int k = 0; k < SR; ++k) {
+        if (k < nr) *o = v[k];
+        o += gx;
+      }
+      if (xe || z == 0 || z == nz - 1) {
+#pragma unroll
+        for (int k = 0; k < SR; ++k)
+          if (k < nr && (x == 0 || x == nx - 1 || y0 + k == 0 || y0 + k == ny - 1 || z == 0 || z == nz - 1))
+            store_images_only(tout, gx, sz, x, y0 + k, z, nx, ny, nz, v[k]);
+      }
+    }
+    out += sz;
+    st = sn;
+  }
+  if (!ok) atomicAdd(&g_bulk_timeouts, 1u);
+}
+
 int check_heat(const nebo_field* T, const nebo_field* To, const nebo_field* L, const char* what) {
   int rc;
   if ((rc = check_field(T, what)) || (rc = check_field(To, what)) || (rc = check_field(L, what))) return rc;
@@ -1112,10 +1248,12 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
       heat_step_kernel<double, ExactD, MODE_REFERENCE><<<grid, block, 0, s>>>(vin.base, vout.base, vl.base, vin.sy,
                                                                               vin.sz, n[0], n[1], n[2], zchunk, p);
   } else {
-    // bulk-copied slabs: rows of 16-byte aligned windows with an even pitch, 8 rows per block
+    // bulk-copied slabs in packed pairs: rows of 16-byte aligned windows with an even pitch, 8 rows
+    // per block.  Its 128 pair columns want wide rows: against the scalar slab kernel below it takes
+    // 45.3 : 56.6 us at 256 columns, 37.0 : 41.1 at 224, 46.4 : 44.7 at 192, 34.9 : 24.6 at 64.
     const int gx = Tf->glob[0], gy = Tf->glob[1];
     const size_t bk_smem = (size_t)BK_NS * 2 * BK_ROWS * gx * sizeof(float) + BK_NS * sizeof(uint64_t);
-    const bool bulk = n[0] <= 2 * BP_PAIRS && n[1] % BK_RY == 0 && gx % 2 == 0 && gy % 2 == 0 &&
+    const bool bulk = n[0] > 192 && n[0] <= 2 * BP_PAIRS && n[1] % BK_RY == 0 && gx % 2 == 0 && gy % 2 == 0 &&
                       (uintptr_t)Tf->data % 16 == 0 && (uintptr_t)Lf->data % 16 == 0 && bk_smem <= 113 * 1024;
     if (bulk) {
       // (per device and cheap: the attribute is set on every launch)
@@ -1134,6 +1272,27 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
       kern<<<dim3(yb, (n[2] + zc - 1) / zc), BP_THREADS, bk_smem, s>>>(
           (const float*)Tf->data, vout.base, (const float*)Lf->data, gx, vin.sz, n[0], n[1], n[2], zc, p.w[0], p.w[1],
           p.w[2]);
+      NEBO_LAUNCH_CHECK("nebo_heat_step");
+      return NEBO_OK;
+    }
+    if (n[0] <= SL_MAXX) {
+      const size_t smem = (size_t)SL_NS * 2 * slab_stage_bytes(gx) + SL_NS * sizeof(uint64_t);
+      auto kern = heat_step_f32_slab_kernel;
+      NEBO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const int bx = (n[0] + 31) / 32 * 32, yb = (n[1] + SL_R - 1) / SL_R;
+      int bps = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, bx, smem) != cudaSuccess || bps < 1) {
+        cudaGetLastError();
+        bps = 1;
+      }
+      // one wave of resident blocks, chunks of 3 planes or more
+      const int ch = max(1, min(num_sms() * bps / yb, (n[2] + 2) / 3));
+      const int zc = (n[2] + ch - 1) / ch;
+      const long total = (long)gx * gy * Tf->glob[2];
+      LaunchScope ls("heat_step_f32", s);
+      kern<<<dim3(yb, (n[2] + zc - 1) / zc), bx, smem, s>>>((const float*)Tf->data, vout.base, (const float*)Lf->data,
+                                                            total, gx, vin.sz, n[0], n[1], n[2], zc, p.w[0], p.w[1],
+                                                            p.w[2]);
       NEBO_LAUNCH_CHECK("nebo_heat_step");
       return NEBO_OK;
     }
