@@ -103,19 +103,5 @@ __device__ __forceinline__ void acc4_add(Acc4& a, double v) {
   keys_add(a.mx, a.mn, order_key(v));
 }
 
-// out = {sum, max, min, norm} of the partial accumulators (one block).
-__global__ void __launch_bounds__(256) reduce4_final_kernel(const Acc4* __restrict__ partials, int n,
-                                                                    double* __restrict__ out) {
-  Acc4 a{0.0, 0.0, 0.0, 0.0, LLONG_MIN, LLONG_MAX};
-  for (int i = threadIdx.x; i < n; i += blockDim.x) merge4(a, partials[i]);
-  a = block_reduce4(a);
-  if (threadIdx.x == 0) {
-    out[0] = a.s + a.sc;
-    out[1] = a.mx == LLONG_MIN ? -INFINITY : from_key(a.mx);
-    out[2] = a.mn == LLONG_MAX ? INFINITY : from_key(a.mn);
-    out[3] = sqrt(a.q + a.qc);
-  }
-}
-
 }  // namespace
 }  // namespace nebo
