@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "bulk.cuh"
+#include "softflux.cuh"
 
 struct nebo_patchset;  // opaque handle of the C ABI
 
@@ -174,6 +175,176 @@ __global__ void __launch_bounds__(PT_THREADS) patches_step_kernel(const PatchDev
       fzlo = fzhi;
     }
     __syncthreads();  // shared faces are reused by the next item
+  }
+}
+
+// One persistent launch = one FP64 time step of every patch, the x and y face fluxes on the integer
+// pipe (soft_flux, softflux.cuh; lambda is one s = 2 lambda per patch) beside the FP64 z flux and
+// update, arranged as in heat_soft.cuh: values are unpacked once and staged with their halo two
+// planes ahead, the update of plane z runs beside the integer fluxes of plane z + 1.  The same bits
+// as FP64 fluxes: 9 FP64 operations per cell instead of 13, which is what bounds the step (with the
+// lanes that a tile's ragged edge leaves idle).  128 patches of 16..96 cells an edge: 816 -> 612 us
+// per step; z chunks of 16 planes (32: 608, but 20 small patches 47 -> 58).
+template <int LX>
+struct PatchSoftShared {
+  static constexpr int TX = 1 << LX, TY = PT_THREADS >> LX, W = TX + 2;
+  long long m[2][(TY + 2) * W];
+  int e[2][(TY + 2) * W];
+  double fx[2][TY * (TX + 1)];
+  double fy[2][(TY + 1) * TX];
+};
+union PatchSoftAny {
+  PatchSoftShared<4> s4;
+  PatchSoftShared<5> s5;
+  PatchSoftShared<6> s6;
+};
+
+template <int LX>
+__device__ __forceinline__ void patch_soft_item(PatchSoftShared<LX>& sm, const PatchDev& P, const WorkItem& it,
+                                                const double* __restrict__ src, double* __restrict__ dst) {
+  constexpr int TX = 1 << LX, TY = PT_THREADS >> LX, W = TX + 2;
+  using softfp::SoftVal;
+  const int tid = threadIdx.x, tx = tid & (TX - 1), ty = tid >> LX;
+  const int nx = P.nx, ny = P.ny, nz = P.nz, sy = nx + 2, sz = (nx + 2) * (ny + 2);
+  const double s = P.lam2, hdt = P.hdt;
+  const double* tin = src + P.offset + 1 + sy + sz;  // interior (0, 0, 0)
+  double* tout = dst + P.offset + 1 + sy + sz;
+  const int x0 = it.x0, y0 = it.y0, z0 = it.z0, z1 = it.z1;
+  const int ic = min(x0 + tx, nx) + sy * min(y0 + ty, ny);
+  const int si = (ty + 1) * W + tx + 1;
+  auto hard = [&](SoftVal a, SoftVal b) { return __dmul_rn(s, __dsub_rn(softfp::pack(b), softfp::pack(a))); };
+  auto stage = [&](int buf, int i, double t) {
+    const SoftVal v = softfp::unpack(t);
+    sm.m[buf][i] = v.m;
+    sm.e[buf][i] = v.e;
+    return v;
+  };
+  auto staged = [&](int buf, int i) {
+    SoftVal v;
+    v.m = sm.m[buf][i];
+    v.e = sm.e[buf][i];
+    return v;
+  };
+  // halo cells, from thread 64 on: columns x0 + TX and x0 - 1, rows y0 - 1 and y0 + TY (clamped into
+  // the window; a clamped cell feeds no active face)
+  const int h = tid - 64;
+  const bool halo = h >= 0 && h < 2 * TY + 2 * TX;
+  int ih, hi;
+  if (h < 2 * TY) {
+    const int r = h & (TY - 1);
+    ih = (h < TY ? min(x0 + TX, nx) : x0 - 1) + sy * min(y0 + r, ny);
+    hi = (r + 1) * W + (h < TY ? TX + 1 : 0);
+  } else {
+    const int c = (h - 2 * TY) & (TX - 1), up = (h - 2 * TY) >> LX;
+    ih = min(x0 + c, nx) + sy * (up ? min(y0 + TY, ny) : y0 - 1);
+    hi = (up ? (TY + 1) * W : 0) + c + 1;
+  }
+  // the extra faces: the first TX threads those above the tile, the next TY those right of it
+  const bool up = tid < TX;
+  const bool xface = up ? (y0 + TY <= ny && x0 + tid <= nx)
+                        : (tid < TX + TY && x0 + TX <= nx && y0 + (tid - TX) < ny);
+  auto extra = [&](int buf) {
+    if (xface) {
+      const int i = up ? TY * W + tid + 1 : (tid - TX + 1) * W + TX;
+      const SoftVal a = staged(buf, i), b = staged(buf, i + (up ? W : 1));
+      bool ok;
+      double f = softfp::soft_flux(s, a, b, ok);
+      if (!ok) f = hard(a, b);
+      *(up ? &sm.fy[buf][TY * TX + tid] : &sm.fx[buf][(tid - TX) * (TX + 1) + TX]) = f;
+    }
+  };
+  double tc, tn, tn2, fzlo, fzhi, fx, fy;
+  SoftVal X;  // of plane z + 1
+  {
+    const double* t0 = tin + (long)sz * z0;
+    tc = __ldg(t0 + ic);
+    tn = __ldg(t0 + sz + ic);
+    const double tm = __ldg(t0 - sz + ic);
+    fzlo = __dmul_rn(s, __dsub_rn(tc, tm));
+    fzhi = __dmul_rn(s, __dsub_rn(tn, tc));
+    const int b = z0 & 1;
+    const SoftVal X0 = stage(b, si, tc);
+    X = stage(b ^ 1, si, tn);
+    if (halo) {
+      stage(b, hi, __ldg(t0 + ih));
+      stage(b ^ 1, hi, __ldg(t0 + sz + ih));
+    }
+    __syncthreads();
+    bool ok;
+    const SoftVal ax = staged(b, si - 1);
+    fx = softfp::soft_flux(s, ax, X0, ok);
+    if (!ok) fx = hard(ax, X0);
+    const SoftVal ay = staged(b, si - W);
+    fy = softfp::soft_flux(s, ay, X0, ok);
+    if (!ok) fy = hard(ay, X0);
+    sm.fx[b][ty * (TX + 1) + tx] = fx;
+    sm.fy[b][ty * TX + tx] = fy;
+    extra(b);
+    tn2 = __ldg(tin + (long)sz * min(z0 + 2, nz) + ic);
+  }
+  auto store = [&](int z, double v) {
+    const int x = x0 + tx, y = y0 + ty;
+    if (x < nx && y < ny) store_images(tout, sy, (long)sz, x, y, z, nx, ny, nz, v);
+  };
+#pragma unroll 1
+  for (int z = z0;; ++z) {
+    __syncthreads();
+    const int buf = z & 1, nb = buf ^ 1;
+    const double a = __dsub_rn(sm.fx[buf][ty * (TX + 1) + tx + 1], fx);
+    const double b = __dsub_rn(sm.fy[buf][(ty + 1) * TX + tx], fy);
+    const double c = __dsub_rn(fzhi, fzlo);
+    if (z + 1 >= z1) {
+      store(z, __dadd_rn(tc, __dmul_rn(hdt, __dadd_rn(__dadd_rn(a, b), c))));
+      break;
+    }
+    const double dz = __dsub_rn(tn2, tn);
+    const SoftVal xl = staged(nb, si - 1);
+    bool okx, oky;
+    double gx = softfp::soft_flux(s, xl, X, okx);
+    const double ab = __dadd_rn(a, b);
+    const SoftVal yl = staged(nb, si - W);
+    double gy = softfp::soft_flux(s, yl, X, oky);
+    const double sum = __dadd_rn(ab, c);
+    // plane z + 2 (exists: z + 1 < z1 <= nz)
+    const SoftVal Xn = stage(buf, si, tn2);
+    if (halo) stage(buf, hi, __ldg(tin + (long)sz * (z + 2) + ih));
+    const double prod = __dmul_rn(hdt, sum);
+    const double gz = __dmul_rn(s, dz);
+    const double v = __dadd_rn(tc, prod);
+    if (!(okx && oky)) {
+      gx = hard(xl, X);
+      gy = hard(yl, X);
+    }
+    sm.fx[nb][ty * (TX + 1) + tx] = gx;
+    sm.fy[nb][ty * TX + tx] = gy;
+    extra(nb);
+    tc = tn;
+    tn = tn2;
+    tn2 = __ldg(tin + (long)sz * min(z + 3, nz) + ic);  // past nz: read again, not used
+    store(z, v);
+    fx = gx;
+    fy = gy;
+    fzlo = fzhi;
+    fzhi = gz;
+    X = Xn;
+  }
+}
+
+__global__ void __launch_bounds__(PT_THREADS, 4) patches_soft_kernel(const PatchDev* __restrict__ patches,
+                                                                     const WorkItem* __restrict__ items, int nitems,
+                                                                     const double* __restrict__ src,
+                                                                     double* __restrict__ dst) {
+  __shared__ PatchSoftAny sm;
+  for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
+    const WorkItem it = items[w];
+    const PatchDev P = patches[it.patch];
+    if (P.log2tx == 4)
+      patch_soft_item<4>(sm.s4, P, it, src, dst);
+    else if (P.log2tx == 5)
+      patch_soft_item<5>(sm.s5, P, it, src, dst);
+    else
+      patch_soft_item<6>(sm.s6, P, it, src, dst);
+    __syncthreads();  // the staged planes and faces are reused by the next item
   }
 }
 
@@ -527,6 +698,7 @@ struct PatchSet {
   int nitems = 0;
   int zchunk = 16;
   int grid = 0;
+  bool wide_plane = false;  // some patch plane holds 2^31 cells or more (64-bit offsets: patches_step_kernel)
   int grid32 = 0;  // resident blocks of the FP32 ring kernel (one full wave)
   bool bulk32 = false;            // FP32 mode on the slab layout (every nx <= PB_CELLS)
   std::vector<long long> off32;   // slab layout: interior offsets
@@ -602,10 +774,13 @@ int launch_step(const PatchSet& ps, const WorkItem* items, int nitems, int parit
   if (nitems == 0) return NEBO_OK;
   LaunchScope ls(ps.dtype == NEBO_F64 ? "patches_step_f64" : (ps.dtype == NEBO_F32 ? "patches_step_f32" : "patches_step_f32x2"), s);
   const int grid = std::min(nitems, ps.grid);
-  if (ps.dtype == NEBO_F64)
+  if (ps.dtype == NEBO_F64 && ps.wide_plane)
     patches_step_kernel<PMODE_F64><<<grid, PT_THREADS, 0, s>>>(ps.d_patches, items, nitems,
                                                                (const double*)ps.arena[parity],
                                                                (double*)ps.arena[parity ^ 1]);
+  else if (ps.dtype == NEBO_F64)
+    patches_soft_kernel<<<grid, PT_THREADS, 0, s>>>(ps.d_patches, items, nitems, (const double*)ps.arena[parity],
+                                                    (double*)ps.arena[parity ^ 1]);
   else if (ps.dtype == NEBO_F32 && ps.bulk32)
     patches_f32_bulk_kernel<<<std::min(nitems, ps.grid32), PT_THREADS,
                               (size_t)PB_NS * ps.stage32 * sizeof(float) + PB_NS * sizeof(uint64_t), s>>>(
@@ -672,6 +847,7 @@ extern "C" int nebo_patchset_create(nebo_patchset** out, int npatch, const int32
       return fail(NEBO_ERR_INVALID, "Nebo error in nebo_patchset_create: patch %d has an edge below 2", p);
     }
     ps->offset[p] = off;
+    ps->wide_plane = ps->wide_plane || (long long)(nx + 2) * (ny + 2) >= (1LL << 31);
     off += (long long)(nx + 2) * (ny + 2) * (nz + 2);
     off = (off + 31) & ~31LL;  // 256-byte aligned windows
     ps->log2tx[p] = default_log2tx(nx);
