@@ -99,6 +99,16 @@ int heat_step_faces(const nebo_field* T, const nebo_field* To, const double* con
                     const double sp[3], cudaStream_t s);
 bool heat_faces_ok(const nebo_field* f);
 
+// Whether work enqueued on s is being recorded into a graph by the caller.
+inline bool stream_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 // SM count of the current device, queried once (callers on several threads may race to the
 // first query; they store the same value).
 inline int num_sms() {

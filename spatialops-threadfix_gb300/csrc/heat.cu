@@ -1488,16 +1488,6 @@ bool heat_faces_ok(const nebo_field* f) { return (long)f->glob[0] * f->glob[1] <
 
 namespace {
 
-// Whether work enqueued on s is being recorded into a graph by the caller.
-bool capturing(cudaStream_t s) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-    cudaGetLastError();
-    return true;
-  }
-  return st != cudaStreamCaptureStatusNone;
-}
-
 // The steps of nebo_heat_run one launch at a time (T's ghosts filled): FP64 on face coefficients in
 // scratch of three fields when `soft`, else (or when the scratch does not fit) on lambda.
 int heat_run_steps(const nebo_field* T, const nebo_field* Ttmp, const nebo_field* lam, int steps, double dt,
@@ -1607,7 +1597,7 @@ extern "C" int nebo_heat_run(const nebo_field* T, const nebo_field* Ttmp, const 
   // more than 1 GB in a cached graph are launched step by step: their steps are long enough.
   const size_t scratch = 3 * (size_t)T->glob[0] * T->glob[1] * T->glob[2] * sizeof(double);
   const bool soft =
-      T->dtype == NEBO_F64 && steps >= (heat_unit(sp) ? 3 : 2) && heat_faces_ok(T) && !capturing(s);
+      T->dtype == NEBO_F64 && steps >= (heat_unit(sp) ? 3 : 2) && heat_faces_ok(T) && !stream_capturing(s);
   if (soft) pool_retain();  // a pool setting: not from inside the capture below
   if (!use_graph || (soft && scratch > (1ul << 30))) return heat_run_steps(T, Ttmp, lam, steps, dt, sp, soft, s);
   GraphKey key{T->data, Ttmp->data, lam->data, {T->glob[0], T->glob[1], T->glob[2]}, T->dtype, steps, soft ? -2 : -1,

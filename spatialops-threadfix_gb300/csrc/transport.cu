@@ -94,10 +94,11 @@ __device__ __forceinline__ void store_images2(T* base, int sy, long sz, int x, i
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 constexpr int PFZ = 6;
 
-template <typename T, bool SECOND>
-__global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<T> a, int zchunk) {
-  __shared__ T sfx[2][TY][TX + 1];
-  __shared__ T sfy[2][TY + 1][TX];
+// FP32 stage for odd pitches or fields that are not 8-byte aligned.
+template <bool SECOND>
+__global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<float> a, int zchunk) {
+  __shared__ float sfx[2][TY][TX + 1];
+  __shared__ float sfy[2][TY + 1][TX];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
   const int n = a.n;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<T> a, in
   const int sy = a.sy;
   const long sz = a.sz;
   auto at = [&](int i, int j, int k) { return (long)i + (long)sy * j + sz * k; };
-  T fzlo = face_flux(a, at(xc, yc, z0), sz, a.w);
+  float fzlo = face_flux(a, at(xc, yc, z0), sz, a.w);
   for (int z = z0; z < z1; ++z) {
     const int buf = z & 1;
     const long c = at(xc, yc, z);
@@ -126,9 +127,9 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<T> a, in
         if (SECOND) prefetch_l2(a.base + cp);
       }
     }
-    const T fzhi = face_flux(a, c + sz, sz, a.w);
-    const T fx = face_flux(a, c, 1, a.u);
-    const T fy = face_flux(a, c, sy, a.v);
+    const float fzhi = face_flux(a, c + sz, sz, a.w);
+    const float fx = face_flux(a, c, 1, a.u);
+    const float fy = face_flux(a, c, sy, a.v);
     sfx[buf][ty][tx] = fx;
     sfy[buf][ty][tx] = fy;
     if (ty == 0) {
@@ -140,26 +141,138 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<T> a, in
     }
     __syncthreads();
     if (active) {
-      const T rhs = ((sfx[buf][ty][tx + 1] - fx) + (sfy[buf][ty + 1][tx] - fy)) + (fzhi - fzlo);
-      // FP32 mode: the float <-> double conversions from the bits (a hardware conversion issues
+      const float rhs = ((sfx[buf][ty][tx + 1] - fx) + (sfy[buf][ty + 1][tx] - fy)) + (fzhi - fzlo);
+      // the float <-> double conversions from the bits (a hardware conversion issues
       // on the FP64 pipe, at the FP64 rate)
-      double rd;
-      if constexpr (sizeof(T) == 4) rd = fixmath::f32_to_f64(rhs); else rd = rhs;
+      const double rd = fixmath::f32_to_f64(rhs);
       double r;
       if (!SECOND)
         r = a.acc[c] + a.dt * rd;
       else
         r = 0.5 * a.base[c] + 0.5 * (a.acc[c] + a.dt * rd);
-      T rs;
-      if constexpr (sizeof(T) == 4) rs = fixmath::f64_to_f32_rn(r); else rs = r;
-      if (a.outS) {
-        a.out64[c] = r;
-        store_images2(a.outS, sy, sz, x, y, z, n, rs);
-      } else {
-        store_images2(reinterpret_cast<T*>(a.out64), sy, sz, x, y, z, n, rs);
-      }
+      a.out64[c] = r;
+      store_images2(a.outS, sy, sz, x, y, z, n, fixmath::f64_to_f32_rn(r));
     }
     fzlo = fzhi;
+  }
+}
+
+// FP64 stage.  Per face, with d1 = phi[f] - phi[f-s] and d3 = phi[f+s] - phi[f-2s],
+//   F = k (27 d1 - d3) - u up,   k = nu (lambda[f-s] + lambda[f]) / 48:
+// 5 FP64 operations (two more where k is not precomputed), the upwind value picked by u's bits; the
+// low x and y faces come from each thread and the high ones through shared memory, the z face and
+// the column's phi window (z - 1 .. z + 2) stay in registers.  The halving of the second stage is an
+// exponent step.  What bounds it: the FP64 pipe at 23 operations per cell (40 in the form that sums
+// the four weighted values and compares u in FP64), 79 % busy: 188 -> 107 us per stage at 127^3.
+// Error against 80-bit arithmetic after 20 steps: 1.15e-16 (2-norm), as before (1.16e-16).
+template <bool SECOND, bool KF>
+__global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<double> a,
+                                                                        const double* __restrict__ kfx,
+                                                                        const double* __restrict__ kfy,
+                                                                        const double* __restrict__ kfz, double kc,
+                                                                        int zchunk) {
+  __shared__ double sfx[2][TY][TX + 1];
+  __shared__ double sfy[2][TY + 1][TX];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+  const int n = a.n, sy = a.sy;
+  const long sz = a.sz;
+  const int x = x0 + tx, y = y0 + ty;
+  const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, n);
+  const bool active = x < n && y < n;
+  const int xc = min(x, n), yc = min(y, n);  // column/row n is a ghost: valid memory
+  auto positive = [](double u) { return __double_as_longlong(u) > 0; };
+  auto coef = [&](const double* kf, long f, long s) {
+    return KF ? __ldg(kf + f) : kc * (__ldg(a.lam + f - s) + __ldg(a.lam + f));
+  };
+  auto flux = [&](double k, double u, double pm2, double pm1, double p0, double pp1) {
+    const double g = fma(27.0, p0 - pm1, pm2 - pp1);
+    return fma(-u, positive(u) ? pm1 : p0, k * g);
+  };
+  auto flux_at = [&](const double* kf, const double* vel, long f, long s) {
+    const double* p = a.phi + f;
+    return flux(coef(kf, f, s), __ldg(vel + f), __ldg(p - 2 * s), __ldg(p - s), __ldg(p), __ldg(p + s));
+  };
+  // the extra faces: warp 0 those above the tile, lanes 0..7 of warp 1 those right of it
+  const bool xface = (ty == 0 && y0 + TY <= n && x <= n) || (ty == 1 && tx < TY && x0 + TX <= n && y0 + tx < n);
+  const long c0 = (long)xc + (long)sy * yc;
+  const long ce = ty == 0 ? (long)xc + (long)sy * (y0 + TY) : (long)(x0 + TX) + (long)sy * (y0 + tx);
+  long c = c0 + sz * z0;
+  double pm1 = __ldg(a.phi + c - sz), p0 = __ldg(a.phi + c), p1 = __ldg(a.phi + c + sz);
+  double fzlo = flux(coef(kfz, c, sz), __ldg(a.w + c), __ldg(a.phi + c - 2 * sz), pm1, p0, p1);
+#pragma unroll 1
+  for (int z = z0; z < z1; ++z, c += sz) {
+    const int buf = z & 1;
+    {
+      // the planes this column reads first at step z + PFZ (clamped inside the window)
+      const int zp = min(z + PFZ, n + 1);
+      const long cp = c0 + sz * zp;
+      prefetch_l2(a.phi + cp);
+      if (KF) {
+        if (zp <= n) {
+          prefetch_l2(kfx + cp);
+          prefetch_l2(kfy + cp);
+          prefetch_l2(kfz + cp);
+        }
+      } else {
+        prefetch_l2(a.lam + cp);
+      }
+      prefetch_l2(a.u + cp);
+      prefetch_l2(a.v + cp);
+      prefetch_l2(a.w + cp);
+      if (zp < n) {
+        if (SECOND) prefetch_l2(a.base + cp);
+      }
+    }
+    const double p2 = __ldg(a.phi + c + 2 * sz);
+    const double base = SECOND ? a.base[c] : 0.0;
+    const double fx = flux(coef(kfx, c, 1), __ldg(a.u + c), __ldg(a.phi + c - 2), __ldg(a.phi + c - 1), p0,
+                           __ldg(a.phi + c + 1));
+    const double fy = flux(coef(kfy, c, sy), __ldg(a.v + c), __ldg(a.phi + c - 2 * sy), __ldg(a.phi + c - sy), p0,
+                           __ldg(a.phi + c + sy));
+    sfx[buf][ty][tx] = fx;
+    sfy[buf][ty][tx] = fy;
+    if (xface) {
+      const long f = ce + sz * z;
+      if (ty == 0)
+        sfy[buf][TY][tx] = flux_at(kfy, a.v, f, sy);
+      else
+        sfx[buf][tx][TX] = flux_at(kfx, a.u, f, 1);
+    }
+    const double fzhi = flux(coef(kfz, c + sz, sz), __ldg(a.w + c + sz), pm1, p0, p1, p2);
+    const double dz = fzhi - fzlo;
+    __syncthreads();
+    if (active) {
+      const double rhs = ((sfx[buf][ty][tx + 1] - fx) + (sfy[buf][ty + 1][tx] - fy)) + dz;
+      double r = fma(a.dt, rhs, p0);  // FP64 stages advance from the state they read
+      if (SECOND) {
+        r = base + r;
+        const long long b = __double_as_longlong(r);
+        const int e = (int)((b >> 52) & 0x7ff);
+        r = e >= 2 && e < 0x7ff ? __longlong_as_double(b - (1LL << 52)) : 0.5 * r;
+      }
+      store_images2(a.out64, sy, sz, x, y, z, n, r);
+    }
+    fzlo = fzhi;
+    pm1 = p0;
+    p0 = p1;
+    p1 = p2;
+  }
+}
+
+// k of every face of the stages above (cells 0 .. n of each axis: n is the high face of the last
+// cell, and the tiles' idle lanes read there).
+__global__ void __launch_bounds__(TX* TY) transport_coef_kernel(const double* __restrict__ L, double* __restrict__ kfx,
+                                                                double* __restrict__ kfy, double* __restrict__ kfz,
+                                                                int sy, long sz, int n, double kc) {
+  const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+  if (x > n || y > n) return;
+  for (int z = blockIdx.z; z <= n; z += gridDim.z) {
+    const long c = (long)x + (long)sy * y + sz * z;
+    const double l = __ldg(L + c);
+    kfx[c] = kc * (__ldg(L + c - 1) + l);
+    kfy[c] = kc * (__ldg(L + c - sy) + l);
+    kfz[c] = kc * (__ldg(L + c - sz) + l);
   }
 }
 
@@ -539,6 +652,27 @@ int cast_f64_to_f32(const double* a, float* b, size_t n, cudaStream_t s) {
   return NEBO_OK;
 }
 
+// One FP64 stage; kf: transport_coef_kernel's arrays or null.
+int transport_launch_f64(const TrArgs<double>& a, const double* const kf[3], double kc, bool second, cudaStream_t s) {
+  const int n = a.n, gxb = (n + TX - 1) / TX, gyb = (n + TY - 1) / TY;
+  static std::atomic<int> per_sm[2][2];  // zero: not queried
+  std::atomic<int>& cache = per_sm[kf[0] != nullptr][second];
+  auto go = [&](auto kern) {
+    // z chunks in whole waves of resident blocks (a chunk reads 2G halo planes beyond its own)
+    const int zchunk =
+        wave_zchunk((long)gxb * gyb, (long)num_sms() * blocks_per_sm(kern, TX * TY, cache), n, 2 * G, 8, 1);
+    LaunchScope ls("transport_stage_f64", s);
+    kern<<<dim3(gxb, gyb, (n + zchunk - 1) / zchunk), dim3(TX, TY), 0, s>>>(a, kf[0], kf[1], kf[2], kc, zchunk);
+  };
+  if (kf[0]) {
+    if (second) go(transport_stage_f64_kernel<true, true>); else go(transport_stage_f64_kernel<false, true>);
+  } else {
+    if (second) go(transport_stage_f64_kernel<true, false>); else go(transport_stage_f64_kernel<false, false>);
+  }
+  NEBO_LAUNCH_CHECK("nebo_transport_run");
+  return NEBO_OK;
+}
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -573,8 +707,7 @@ bool window_map(CUtensorMap* m, const float* base, int gl) {
 }
 
 // maps: the tensor maps of a.phi's and a.lam's windows, or nullptr (no tensor staging)
-template <typename T>
-int transport_launch(TrArgs<T> a, bool second, cudaStream_t s, const TrMaps* maps = nullptr) {
+int transport_launch(TrArgs<float> a, bool second, cudaStream_t s, const TrMaps* maps) {
   const int n = a.n;
   const int gxb = (n + TX - 1) / TX, gyb = (n + TY - 1) / TY;
   // FP32 kernels: 3 = cell pairs with tensor-tile staging (kind 2 and tensor maps), 2 = cell
@@ -582,7 +715,7 @@ int transport_launch(TrArgs<T> a, bool second, cudaStream_t s, const TrMaps* map
   // lambda 8-byte aligned), 0 = the generic kernel
   auto al8 = [](const void* p) { return ((uintptr_t)p & 7u) == 0; };
   int kind = 0;
-  if (sizeof(T) == 4 && a.sy % 2 == 0 && al8(a.phi) && al8(a.lam)) {
+  if (a.sy % 2 == 0 && al8(a.phi) && al8(a.lam)) {
     kind = 1;
     if (al8(a.u) && al8(a.v) && al8(a.w) && al8(a.outS)) kind = maps ? 3 : 2;
   }
@@ -600,12 +733,12 @@ int transport_launch(TrArgs<T> a, bool second, cudaStream_t s, const TrMaps* map
     ps = second ? blocks_per_sm(transport_stage_f32_staged_kernel<true>, TX * TY, cache)
                 : blocks_per_sm(transport_stage_f32_staged_kernel<false>, TX * TY, cache);
   else
-    ps = second ? blocks_per_sm(transport_stage_kernel<T, true>, TX * TY, cache)
-                : blocks_per_sm(transport_stage_kernel<T, false>, TX * TY, cache);
+    ps = second ? blocks_per_sm(transport_stage_kernel<true>, TX * TY, cache)
+                : blocks_per_sm(transport_stage_kernel<false>, TX * TY, cache);
   const int zchunk = wave_zchunk((long)gxb * gyb, (long)num_sms() * ps, n, 2 * G, 8, 1);
   dim3 grid(gxb, gyb, (n + zchunk - 1) / zchunk), block(TX, TY);
-  LaunchScope ls(sizeof(T) == 4 ? "transport_stage_f32" : "transport_stage_f64", s);
-  if constexpr (sizeof(T) == 4) {
+  LaunchScope ls("transport_stage_f32", s);
+  {
     if (kind == 3) {
       if (second)
         transport_stage_f32_pair_kernel<true, true><<<grid, dim3(PTX, TY), 0, s>>>(a, zchunk, *maps);
@@ -633,9 +766,9 @@ int transport_launch(TrArgs<T> a, bool second, cudaStream_t s, const TrMaps* map
     }
   }
   if (second)
-    transport_stage_kernel<T, true><<<grid, block, 0, s>>>(a, zchunk);
+    transport_stage_kernel<true><<<grid, block, 0, s>>>(a, zchunk);
   else
-    transport_stage_kernel<T, false><<<grid, block, 0, s>>>(a, zchunk);
+    transport_stage_kernel<false><<<grid, block, 0, s>>>(a, zchunk);
   NEBO_LAUNCH_CHECK("nebo_transport_run");
   return NEBO_OK;
 }
@@ -699,29 +832,42 @@ extern "C" int nebo_transport_run(double* phi, const void* u, const void* v, con
     a.n = n;
     a.sy = (int)sy;
     a.sz = sz;
-    a.nu = nu;
-    const double h = 1.0 / 24.0;
-    a.q0 = h;
-    a.q1 = -27.0 * h;
-    a.q2 = 27.0 * h;
-    a.q3 = -h;
     a.dt = dt;
+    const double kc = nu / 48.0;
+    // The face coefficients once per run, in scratch of three fields, where they pay (their pass
+    // costs about a fifth of a stage and saves an eighth of each) and the caller records no graph;
+    // without them every stage forms them.
+    const double* kf[3] = {nullptr, nullptr, nullptr};
+    double* scratch = nullptr;
+    if (steps >= 2 && !stream_capturing(s)) {
+      pool_retain();
+      if (cudaMallocAsync((void**)&scratch, 3 * cells * sizeof(double), s) != cudaSuccess) {
+        cudaGetLastError();
+        scratch = nullptr;
+      }
+    }
+    if (scratch) {
+      double* out[3];
+      for (int d = 0; d < 3; ++d) kf[d] = out[d] = scratch + d * cells + interior;
+      LaunchScope ls("transport_coef", s);
+      transport_coef_kernel<<<dim3((n + TX) / TX, (n + TY) / TY, n < 63 ? n + 1 : 64), dim3(TX, TY), 0, s>>>(
+          a.lam, out[0], out[1], out[2], a.sy, a.sz, n, kc);
+    }
     double* cur = phi;
-    for (int k = 0; k < steps; ++k) {
+    for (int k = 0; k < steps && !rc; ++k) {
       // stage 1: phi1 = cur + dt R(cur)
       a.phi = cur + interior;
-      a.acc = cur + interior;
       a.out64 = phi1 + interior;
-      a.outS = nullptr;
-      if ((rc = transport_launch(a, false, s))) return rc;
+      if ((rc = transport_launch_f64(a, kf, kc, false, s))) break;
       // stage 2: phin = cur/2 + (phi1 + dt R(phi1))/2
       a.phi = phi1 + interior;
-      a.acc = phi1 + interior;
       a.base = cur + interior;
       a.out64 = (cur == phi ? phin : phi) + interior;
-      if ((rc = transport_launch(a, true, s))) return rc;
+      rc = transport_launch_f64(a, kf, kc, true, s);
       cur = (cur == phi) ? phin : phi;
     }
+    if (scratch) cudaFreeAsync(scratch, s);
+    if (rc) return rc;
     if (cur != phi) NEBO_CUDA_TRY(cudaMemcpyAsync(phi, cur, cells * sizeof(double), cudaMemcpyDeviceToDevice, s));
     return NEBO_OK;
   }
