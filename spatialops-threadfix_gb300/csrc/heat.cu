@@ -691,20 +691,72 @@ __global__ void fxs_setup_kernel(FxState* c, double w) {
   c->M[0] = c->M[1] = c->M[2] = 0ull;
 }
 
-// largest biased exponent of lambda -> atomicMax(c->eL); any lambda < 0 -> c->negL = 1
-__global__ void fxs_lambda_scan_kernel(const double* __restrict__ f, long n, FxState* __restrict__ c) {
-  int m = 0, neg = 0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const double v = f[i];
-    m = max(m, (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ff));
-    neg |= v < 0.0;
-  }
-  m = __reduce_max_sync(0xffffffffu, m);
+// The passes before and after the steps read or write whole windows; four loads in flight per
+// thread and integer conversions leave them to HBM (256^3: scan, conversion and the way back 202 us;
+// one load in flight and FP64 conversions, ldexp among them, 623).
+template <class F>
+__device__ __forceinline__ void four_each(long n, F&& f) {
+  const long step = (long)gridDim.x * blockDim.x;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += 4 * step) f(i, step);
+}
+
+// largest biased exponents of T and of lambda -> atomicMax(c->eT, c->eL); any lambda < 0 -> negL = 1
+__global__ void __launch_bounds__(256) fxs_scan_kernel(const double* __restrict__ t, const double* __restrict__ l,
+                                                       long n, FxState* __restrict__ c) {
+  int mt = 0, ml = 0, neg = 0;
+  four_each(n, [&](long i, long step) {
+    long long a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      a[k] = i + k * step < n ? __double_as_longlong(__ldg(t + i + k * step)) : 0;
+      b[k] = i + k * step < n ? __double_as_longlong(__ldg(l + i + k * step)) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      mt = max(mt, (int)(a[k] >> 52) & 0x7ff);
+      ml = max(ml, (int)(b[k] >> 52) & 0x7ff);
+      neg |= b[k] < 0 && (b[k] << 1) != 0;  // -0 is no negative value; a NaN takes the exact form anyway
+    }
+  });
+  mt = __reduce_max_sync(0xffffffffu, mt);
+  ml = __reduce_max_sync(0xffffffffu, ml);
   neg = __reduce_or_sync(0xffffffffu, neg);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(&c->eL, m);
+    atomicMax(&c->eT, mt);
+    atomicMax(&c->eL, ml);
     if (neg) atomicOr(&c->negL, 1);
   }
+}
+
+// RN(v 2^s) as an integer (ties to even), |v 2^s| < 2^63.
+__device__ __forceinline__ long long scaled_ll(double v, int s) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const int ef = (int)((b >> 52) & 0x7ff);
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (ef ? 1ull << 52 : 0ull);
+  const int sh = (ef ? ef : 1) - 1075 + s;
+  unsigned long long r;
+  if (sh >= 0) {
+    r = m << sh;
+  } else if (sh > -55) {
+    const unsigned long long q = m >> -sh, half = 1ull << (-sh - 1), rem = m & ((half << 1) - 1);
+    r = q + (rem > half || (rem == half && (q & 1)) ? 1 : 0);
+  } else {
+    r = 0;
+  }
+  return (long long)b < 0 ? -(long long)r : (long long)r;
+}
+
+// RN(v 2^U) with the result's exponent in the normal range, else ldexp.
+__device__ __forceinline__ double scaled_double(long long v, int U) {
+  const unsigned long long a = (unsigned long long)(v < 0 ? -v : v);
+  const int lz = fixmath::clz64(a), e = 63 - lz + U + 1023;
+  if (a == 0 || e < 2 || e > 2045) return ldexp(__ll2double_rn(v), U);
+  const unsigned long long top = a << lz;
+  unsigned long long m = top >> 11;
+  const unsigned rem = (unsigned)top & 0x7ffu;
+  m += rem > 0x400u || (rem == 0x400u && (m & 1)) ? 1 : 0;
+  return __longlong_as_double((long long)((((unsigned long long)(e - 1) << 52) + m) |
+                                          ((unsigned long long)v & (1ull << 63))));
 }
 
 __device__ __forceinline__ unsigned long long or_warp64(unsigned long long v) {
@@ -714,36 +766,52 @@ __device__ __forceinline__ unsigned long long or_warp64(unsigned long long v) {
 }
 
 // state 0 and the lambda weights (every cell of the windows, ghosts included)
-__global__ void fxs_convert_kernel(const double* __restrict__ t, long long* __restrict__ tfix,
-                                   const double* __restrict__ lam, long long* __restrict__ lw, long n,
-                                   FxState* __restrict__ c, double w) {
+__global__ void __launch_bounds__(256) fxs_convert_kernel(const double* __restrict__ t, long long* __restrict__ tfix,
+                                                          const double* __restrict__ lam, long long* __restrict__ lw,
+                                                          long n, FxState* __restrict__ c, double w) {
   const bool plain = c->plain;
   const int U = c->U[0], k = c->k;
   unsigned long long m = 0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const double tv = t[i], lv = lam[i];
-    if (plain) {
-      tfix[i] = __double_as_longlong(tv);
-      lw[i] = __double_as_longlong(lv);
-    } else {
-      const long long a = __double2ll_rn(ldexp(tv, -U));
-      tfix[i] = a;
-      lw[i] = __double2ll_rn(ldexp(w * lv, 64 - k));
-      m |= (unsigned long long)(a ^ (a >> 63));
+  four_each(n, [&](long i, long step) {
+    double tv[4], lv[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      tv[q] = i + q * step < n ? __ldg(t + i + q * step) : 0.0;
+      lv[q] = i + q * step < n ? __ldg(lam + i + q * step) : 0.0;
     }
-  }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (i + q * step >= n) break;
+      long long a, b;
+      if (plain) {
+        a = __double_as_longlong(tv[q]);
+        b = __double_as_longlong(lv[q]);
+      } else {
+        a = scaled_ll(tv[q], -U);
+        b = scaled_ll(w * lv[q], 64 - k);
+        m |= (unsigned long long)(a ^ (a >> 63));
+      }
+      tfix[i + q * step] = a;
+      lw[i + q * step] = b;
+    }
+  });
   m = or_warp64(m);
   if ((threadIdx.x & 31) == 0 && m) atomicOr(&c->M[0], m);
 }
 
-__global__ void fxs_finish_kernel(const long long* __restrict__ tfix, double* __restrict__ t, long n,
-                                  const FxState* __restrict__ c, int slot) {
+__global__ void __launch_bounds__(256) fxs_finish_kernel(const long long* tfix, double* t, long n,
+                                                         const FxState* __restrict__ c, int slot) {
   const bool plain = c->plain;
   const int U = c->U[slot];
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const long long v = tfix[i];
-    t[i] = plain ? __longlong_as_double(v) : ldexp(__ll2double_rn(v), U);
-  }
+  // tfix and t may be one array: a thread reads its four values before it writes them
+  four_each(n, [&](long i, long step) {
+    long long v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = i + q * step < n ? tfix[i + q * step] : 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i + q * step < n) t[i + q * step] = plain ? __longlong_as_double(v[q]) : scaled_double(v[q], U);
+  });
 }
 
 // One step on a 32 x 8 tile marching z, staged like heat_step_fix_kernel (the tile and its x / y
@@ -901,12 +969,11 @@ int heat_run_fixed_state(const nebo_field* T, const nebo_field* Ttmp, const nebo
     return cuda_fail(err, what);
   }
   const double w = 0.5 * dt;
-  const int rblocks = num_sms() * 4;
+  const int rblocks = num_sms() * 8;
   err = cudaMemsetAsync(c, 0, sizeof(FxState), s);
   if (err == cudaSuccess) {
     LaunchScope ls("heat_fixed_state_in", s);
-    max_biased_exp_kernel<<<rblocks, 256, 0, s>>>((const double*)T->data, cells, &c->eT);
-    fxs_lambda_scan_kernel<<<rblocks, 256, 0, s>>>((const double*)lam->data, cells, c);
+    fxs_scan_kernel<<<rblocks, 256, 0, s>>>((const double*)T->data, (const double*)lam->data, cells, c);
     fxs_setup_kernel<<<1, 1, 0, s>>>(c, w);
     fxs_convert_kernel<<<rblocks, 256, 0, s>>>((const double*)T->data, (long long*)Ttmp->data,
                                                (const double*)lam->data, lw, cells, c, w);

@@ -57,14 +57,6 @@ __host__ __device__ __forceinline__ double pack(SoftVal v) {
   return fixmath::from_bits(neg | (ef << 52) | (m & 0xFFFFFFFFFFFFFull));
 }
 
-__host__ __device__ __forceinline__ int clz32(unsigned a) {
-#ifdef __CUDA_ARCH__
-  return __clz((int)a);
-#else
-  return a ? __builtin_clz(a) : 32;
-#endif
-}
-
 // The high word of (hi:lo) << n for 0 <= n < 32.
 __host__ __device__ __forceinline__ unsigned shl_hi(unsigned hi, unsigned lo, int n) {
 #ifdef __CUDA_ARCH__
@@ -96,7 +88,7 @@ __host__ __device__ __forceinline__ SoftDiff soft_diff(SoftVal a, SoftVal b, int
   const long long S = big - t;  // +-(b - a), |S| < 2^63
   const unsigned long long U = (unsigned long long)(S < 0 ? -S : S);
   const unsigned uh = (unsigned)(U >> 32), ul = (unsigned)U;
-  const int lz = uh ? clz32(uh) : 32 + clz32(ul);  // 1 .. 64
+  const int lz = uh ? fixmath::clz32(uh) : 32 + fixmath::clz32(ul);  // 1 .. 64
   const unsigned long long n = U << (lz - 1);
   const unsigned long long r = n + (0x1ffu + (((unsigned)n >> 10) & 1u));
   SoftDiff d;
