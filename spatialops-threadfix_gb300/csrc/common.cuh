@@ -68,6 +68,11 @@ inline View<T> make_view(const nebo_field& f) {
   return v;
 }
 
+// a / b for a >= 0, b > 0: 32-bit where both fit (a 64-bit division takes about 100 instructions).
+__device__ __forceinline__ long fast_div(long a, int b) {
+  return a >> 32 ? a / b : (long)((unsigned)a / (unsigned)b);
+}
+
 // Counts one kernel launch and, while profiling is on, times it with events on its stream.
 // Construct immediately before the launch; the destructor records the end event.
 class LaunchScope {
@@ -92,6 +97,9 @@ void pool_retain();
 
 // Periodic ghost fill of one uniform-ghost patch (ghost.cu).
 int fill_periodic_any(const nebo_field* f, cudaStream_t s);
+// The same for up to 6 fields of one shape (dtypes may differ) in one launch; only the first is
+// checked.
+int fill_periodic_fields(const nebo_field* const* fs, int count, cudaStream_t s);
 
 // The exact FP64 heat step on face coefficients computed once per lambda (heat.cu).
 int heat_face_coef(const nebo_field* lam, double* const lf[3], bool half, cudaStream_t s);

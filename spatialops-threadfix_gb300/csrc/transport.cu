@@ -640,9 +640,17 @@ __global__ void __launch_bounds__(PTX* TY) transport_stage_f32_pair_kernel(TrArg
   }
 }
 
+// 12 bytes per element: bound by HBM with four loads in flight per thread (324^3: 88 -> 66 us).
 __global__ void cast_f64_f32_kernel(const double* __restrict__ a, float* __restrict__ b, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    b[i] = fixmath::f64_to_f32_rn(a[i]);
+  const size_t step = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += 4 * step) {
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = i + k * step < n ? __ldg(a + i + k * step) : 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * step < n) b[i + k * step] = fixmath::f64_to_f32_rn(v[k]);
+  }
 }
 
 int cast_f64_to_f32(const double* a, float* b, size_t n, cudaStream_t s) {
@@ -816,14 +824,21 @@ extern "C" int nebo_transport_run(double* phi, const void* u, const void* v, con
     f.has_bc[i] = f.bc_extra[i] = 0;
   }
   int rc;
-  if (dtype == NEBO_F64) {
-    f.dtype = NEBO_F64;
-    f.data = phi;
-    if ((rc = fill_periodic_any(&f, s))) return rc;
-    for (const void* q : {u, v, w, lam}) {
-      f.data = const_cast<void*>(q);
-      if ((rc = fill_periodic_any(&f, s))) return rc;
+  // the ghosts of the state and the coefficients, in one launch
+  auto fill_inputs = [&](int coef_dtype) {
+    nebo_field fs[5];
+    const nebo_field* ptr[5];
+    const void* data[5] = {phi, u, v, w, lam};
+    for (int i = 0; i < 5; ++i) {
+      fs[i] = f;
+      fs[i].data = const_cast<void*>(data[i]);
+      fs[i].dtype = i ? coef_dtype : NEBO_F64;
+      ptr[i] = &fs[i];
     }
+    return fill_periodic_fields(ptr, 5, s);
+  };
+  if (dtype == NEBO_F64) {
+    if ((rc = fill_inputs(NEBO_F64))) return rc;
     TrArgs<double> a{};
     a.u = (const double*)u + interior;
     a.v = (const double*)v + interior;
@@ -874,14 +889,7 @@ extern "C" int nebo_transport_run(double* phi, const void* u, const void* v, con
   // FP32 storage: float stencil copies + FP64 accumulators
   float* s0 = reinterpret_cast<float*>(phin + cells);
   float* s1 = s0 + cells;
-  f.dtype = NEBO_F32;
-  for (const void* q : {u, v, w, lam}) {
-    f.data = const_cast<void*>(q);
-    if ((rc = fill_periodic_any(&f, s))) return rc;
-  }
-  f.dtype = NEBO_F64;
-  f.data = phi;
-  if ((rc = fill_periodic_any(&f, s))) return rc;
+  if ((rc = fill_inputs(NEBO_F32))) return rc;
   if ((rc = cast_f64_to_f32(phi, s0, cells, s))) return rc;
   TrArgs<float> a{};
   a.u = (const float*)u + interior;
