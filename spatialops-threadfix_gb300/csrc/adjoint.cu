@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "fp64_int.cuh"
+#include "softflux.cuh"
 
 namespace nebo {
 namespace {
@@ -33,7 +34,8 @@ constexpr int BY = 8;
 
 // A forward state as a double (FP32 states widen exactly).
 __device__ __forceinline__ double to_f64(double v) { return v; }
-__device__ __forceinline__ double to_f64(float v) { return (double)v; }
+__device__ __forceinline__ double to_f64(float v) { return fixmath::f32_to_f64(v); }  // by its bits: a
+// hardware conversion issues on the FP64 pipe
 
 __device__ __forceinline__ void store_images1(double* base, int sy, long sz, int x, int y, int z, int nx, int ny, int nz,
                                               double v) {
@@ -61,7 +63,7 @@ __device__ __forceinline__ void store_images1(double* base, int sy, long sz, int
 // only the fold into glam is FP64: 6 FP64 operations per cell fewer, and the adjoint state A,
 // hence dJ/dT0, is unaffected.
 template <bool EXACT, bool LF, typename S = double>
-__global__ void __launch_bounds__(BX* BY, 4) heat_adjoint_kernel(const S* __restrict__ T, const double* __restrict__ Ain,
+__global__ void __launch_bounds__(BX* BY, sizeof(S) == 4 ? 3 : 4) heat_adjoint_kernel(const S* __restrict__ T, const double* __restrict__ Ain,
                                                               double* __restrict__ Aout, const double* __restrict__ L,
                                                               const double* __restrict__ lfx,
                                                               const double* __restrict__ lfy,
@@ -142,6 +144,189 @@ __global__ void __launch_bounds__(BX* BY, 4) heat_adjoint_kernel(const S* __rest
     }
     dazl = dazh;
     dtzl = dtzh;
+  }
+}
+
+// The reverse step on precomputed face coefficients and FP64 states with the x and y differences on
+// the integer pipe (soft_sub, softflux.cuh), arranged as in heat_soft.cuh: T and A are unpacked once
+// and staged with their halo two planes ahead, and the FP64 chains of plane z run beside the integer
+// differences of plane z + 1 of other warps.  The operations and their order are
+// heat_adjoint_kernel's, the bits too: 16 FP64 operations per cell instead of 20, 98 -> 86 us at
+// 128^3 (three blocks per SM at 76 registers; the differences of T alone, 64 registers: 90 to 93; the
+// differences without their fallback branches, so that chains and integers interleave, 89 at 80
+// registers).
+constexpr int AS_W = BX + 2;
+struct AdjShared {
+  long long m[2][2][(BY + 2) * AS_W];  // [buffer][T, A]
+  int e[2][2][(BY + 2) * AS_W];
+  double ax[2][BY][BX + 1], ay[2][BY + 1][BX];
+  double tx[2][BY][BX + 1], ty[2][BY + 1][BX];
+};
+
+template <bool EXACT>
+__global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
+    const double* __restrict__ T, const double* __restrict__ Ain, double* __restrict__ Aout,
+    const double* __restrict__ lfx, const double* __restrict__ lfy, const double* __restrict__ lfz,
+    double* __restrict__ glam, int sy, int sz, int nx, int ny, int nz, int zchunk, double hdt) {
+  __shared__ AdjShared sm;
+  using softfp::SoftVal;
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int x0 = blockIdx.x * BX, y0 = blockIdx.y * BY;
+  const int z0 = blockIdx.z * zchunk, z1 = min(z0 + zchunk, nz);
+  const int xc = min(x0 + tx, nx), yc = min(y0 + ty, ny);
+  const int ic = xc + sy * yc, si = (ty + 1) * AS_W + tx + 1;
+  auto stage = [&](int buf, int f, int i, double v) {
+    const SoftVal u = softfp::unpack(v);
+    sm.m[buf][f][i] = u.m;
+    sm.e[buf][f][i] = u.e;
+    return u;
+  };
+  auto staged = [&](int buf, int f, int i) {
+    SoftVal v;
+    v.m = sm.m[buf][f][i];
+    v.e = sm.e[buf][f][i];
+    return v;
+  };
+  auto sub = [&](SoftVal a, SoftVal b) {
+    bool ok;
+    double d = softfp::soft_sub(a, b, ok);
+    if (!ok) d = __dsub_rn(softfp::pack(b), softfp::pack(a));
+    return d;
+  };
+  // halo cells: warp 1 the columns x0 + 32 (its first 8 lanes) and x0 - 1 (the next 8), warp 2 the
+  // row below, warp 3 the row above; clamped into the window (a clamped cell feeds no active face)
+  const bool halo = (ty == 1 && tx < 2 * BY) || ty == 2 || ty == 3;
+  int ih, hi;
+  if (ty == 1) {
+    const int r = tx & (BY - 1);
+    ih = (tx < BY ? min(x0 + BX, nx) : x0 - 1) + sy * min(y0 + r, ny);
+    hi = (r + 1) * AS_W + (tx < BY ? BX + 1 : 0);
+  } else {
+    ih = xc + sy * (ty == 2 ? y0 - 1 : min(y0 + BY, ny));
+    hi = (ty == 2 ? 0 : (BY + 1) * AS_W) + tx + 1;
+  }
+  // the extra faces: warp 0 those above the tile, the first lanes of warp 1 those right of it
+  const bool xface = (ty == 0 && y0 + BY <= ny && x0 + tx <= nx) ||
+                     (ty == 1 && tx < BY && x0 + BX <= nx && y0 + tx < ny);
+  auto extra = [&](int buf) {
+    if (xface) {
+      const bool up = ty == 0;
+      const int i = up ? BY * AS_W + tx + 1 : (tx + 1) * AS_W + BX, j = i + (up ? AS_W : 1);
+      *(up ? &sm.ty[buf][BY][tx] : &sm.tx[buf][tx][BX]) = sub(staged(buf, 0, i), staged(buf, 0, j));
+      *(up ? &sm.ay[buf][BY][tx] : &sm.ax[buf][tx][BX]) = sub(staged(buf, 1, i), staged(buf, 1, j));
+    }
+  };
+  // differences across the low x and y faces of a staged plane, into the shared faces
+  double dax, day, dtx, dty;
+  auto faces = [&](int buf, SoftVal t, SoftVal a) {
+    dtx = sub(staged(buf, 0, si - 1), t);
+    dax = sub(staged(buf, 1, si - 1), a);
+    dty = sub(staged(buf, 0, si - AS_W), t);
+    day = sub(staged(buf, 1, si - AS_W), a);
+    sm.tx[buf][ty][tx] = dtx;
+    sm.ax[buf][ty][tx] = dax;
+    sm.ty[buf][ty][tx] = dty;
+    sm.ay[buf][ty][tx] = day;
+    extra(buf);
+  };
+  double tn, an, ac, tn2, an2, dazl, dtzl, dazh, dtzh;
+  SoftVal X, Y;  // T and A of plane z + 1
+  {
+    const double* t0 = T + (long)sz * z0;
+    const double* a0 = Ain + (long)sz * z0;
+    const double tc = __ldg(t0 + ic);
+    ac = __ldg(a0 + ic);
+    tn = __ldg(t0 + sz + ic);
+    an = __ldg(a0 + sz + ic);
+    dazl = ac - __ldg(a0 - sz + ic);
+    dtzl = tc - __ldg(t0 - sz + ic);
+    dazh = an - ac;
+    dtzh = tn - tc;
+    const int b = z0 & 1;
+    const SoftVal X0 = stage(b, 0, si, tc), Y0 = stage(b, 1, si, ac);
+    X = stage(b ^ 1, 0, si, tn);
+    Y = stage(b ^ 1, 1, si, an);
+    if (halo) {
+      stage(b, 0, hi, __ldg(t0 + ih));
+      stage(b, 1, hi, __ldg(a0 + ih));
+      stage(b ^ 1, 0, hi, __ldg(t0 + sz + ih));
+      stage(b ^ 1, 1, hi, __ldg(a0 + sz + ih));
+    }
+    __syncthreads();
+    faces(b, X0, Y0);
+    const long o2 = (long)sz * min(z0 + 2, nz);
+    tn2 = __ldg(T + o2 + ic);
+    an2 = __ldg(Ain + o2 + ic);
+  }
+  const bool active = x0 + tx < nx && y0 + ty < ny;
+  auto chain = [&](double kxl, double kxh, double kyl, double kyh, double kzl, double kzh, double daxh, double dayh) {
+    double s = dazh * kzh;
+    s = fma(-dazl, kzl, s);
+    s = fma(dayh, kyh, s);
+    s = fma(-day, kyl, s);
+    s = fma(daxh, kxh, s);
+    return fma(-dax, kxl, s);
+  };
+  auto products = [&](double daxh, double dayh, double dtxh, double dtyh) {
+    if constexpr (EXACT) {
+      double ps = dtzh * dazh;
+      ps = fma(dtzl, dazl, ps);
+      ps = fma(dtyh, dayh, ps);
+      ps = fma(dty, day, ps);
+      ps = fma(dtxh, daxh, ps);
+      return fma(dtx, dax, ps);
+    } else {
+      using fixmath::f32_trunc;
+      float q = f32_trunc(dtzh) * f32_trunc(dazh);
+      q = fmaf(f32_trunc(dtzl), f32_trunc(dazl), q);
+      q = fmaf(f32_trunc(dtyh), f32_trunc(dayh), q);
+      q = fmaf(f32_trunc(dty), f32_trunc(day), q);
+      q = fmaf(f32_trunc(dtxh), f32_trunc(daxh), q);
+      q = fmaf(f32_trunc(dtx), f32_trunc(dax), q);
+      return fixmath::f32_to_f64(q);
+    }
+  };
+  auto store = [&](int z, double v, double gn) {
+    if (active) {
+      glam[(long)sz * z + ic] = gn;
+      store_images1(Aout, sy, sz, x0 + tx, y0 + ty, z, nx, ny, nz, v);
+    }
+  };
+#pragma unroll 1
+  for (int z = z0;; ++z) {
+    __syncthreads();
+    const int buf = z & 1, nb = buf ^ 1;
+    const long o = (long)sz * z + ic;
+    const double daxh = sm.ax[buf][ty][tx + 1], dayh = sm.ay[buf][ty + 1][tx];
+    const double dtxh = sm.tx[buf][ty][tx + 1], dtyh = sm.ty[buf][ty + 1][tx];
+    const double kzh = __ldg(lfz + o + sz), kzl = __ldg(lfz + o), kyh = __ldg(lfy + o + sy), kyl = __ldg(lfy + o),
+                 kxh = __ldg(lfx + o + 1), kxl = __ldg(lfx + o);
+    const double g = active ? glam[o] : 0.0;
+    const double v = fma(hdt, chain(kxl, kxh, kyl, kyh, kzl, kzh, daxh, dayh), ac);
+    const double gn = fma(-hdt, products(daxh, dayh, dtxh, dtyh), g);
+    const bool more = z + 1 < z1;
+    if (more) {
+      dazl = dazh;
+      dtzl = dtzh;
+      dazh = an2 - an;
+      dtzh = tn2 - tn;
+      faces(nb, X, Y);
+      // plane z + 2 (exists: z + 1 < z1 <= nz)
+      X = stage(buf, 0, si, tn2);
+      Y = stage(buf, 1, si, an2);
+      if (halo) {
+        stage(buf, 0, hi, __ldg(T + (long)sz * (z + 2) + ih));
+        stage(buf, 1, hi, __ldg(Ain + (long)sz * (z + 2) + ih));
+      }
+    }
+    store(z, v, gn);
+    if (!more) break;
+    ac = an;
+    tn = tn2;
+    an = an2;
+    const long o3 = (long)sz * min(z + 3, nz);  // past nz: read again, not used
+    tn2 = __ldg(T + o3 + ic);
+    an2 = __ldg(Ain + o3 + ic);
   }
 }
 
@@ -227,6 +412,24 @@ int adjoint_step_lf(const nebo_field* Tk, const nebo_field* Ain, const nebo_fiel
   const View<S> vt = make_view<S>(*Tk);
   const View<double> va = make_view<double>(*Ain), vo = make_view<double>(*Aout), vg = make_view<double>(*glam);
   const int gxb = (n[0] + BX - 1) / BX, gyb = (n[1] + BY - 1) / BY;
+  if constexpr (std::is_same<S, double>::value) {
+    if (heat_faces_ok(Tk)) {
+      static std::atomic<int> per_sm[2];  // z chunks in whole waves of resident blocks (zero: not queried)
+      auto go = [&](auto kern, std::atomic<int>& cache) {
+        const int zchunk =
+            wave_zchunk((long)gxb * gyb, (long)num_sms() * blocks_per_sm(kern, BX * BY, cache), n[2], 2, 4, 1);
+        LaunchScope ls("heat_adjoint_step", s);
+        kern<<<dim3(gxb, gyb, (n[2] + zchunk - 1) / zchunk), dim3(BX, BY), 0, s>>>(
+            vt.base, va.base, vo.base, lfx, lfy, lfz, vg.base, vt.sy, (int)vt.sz, n[0], n[1], n[2], zchunk, 0.5 * dt);
+      };
+      if (exact)
+        go(heat_adjoint_soft_kernel<true>, per_sm[1]);
+      else
+        go(heat_adjoint_soft_kernel<false>, per_sm[0]);
+      NEBO_LAUNCH_CHECK("nebo_heat_gradient (reverse step)");
+      return NEBO_OK;
+    }
+  }
   static std::atomic<int> per_sm[2];  // z chunks in whole waves of resident blocks (zero: not queried)
   const int bps = exact ? blocks_per_sm(heat_adjoint_kernel<true, true, S>, BX * BY, per_sm[1])
                         : blocks_per_sm(heat_adjoint_kernel<false, true, S>, BX * BY, per_sm[0]);

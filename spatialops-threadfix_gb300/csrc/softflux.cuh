@@ -131,5 +131,17 @@ __host__ __device__ __forceinline__ double soft_flux(double s, SoftVal a, SoftVa
   return f;
 }
 
+// RN(b - a) as a double.  covered = false: an operand of the largest binade, non-finite or -0, or a
+// subnormal result; the caller subtracts in FP64.
+__host__ __device__ __forceinline__ double soft_sub(SoftVal a, SoftVal b, bool& covered) {
+  int E;
+  const SoftDiff d = soft_diff(a, b, E);
+  const bool zero = d.dq == 0;
+  covered = E < 2046 && (zero || d.ed > 0);
+  unsigned long long r = (d.dq >> 10) + ((unsigned long long)(unsigned)(d.ed - 1) << 52);
+  if (zero) r = 0;
+  return fixmath::from_bits(r | (zero ? 0ull : (unsigned long long)(d.sign & 0x80000000u) << 32));
+}
+
 }  // namespace softfp
 }  // namespace nebo

@@ -1,5 +1,5 @@
 // Host check of the integer face flux (csrc/softflux.cuh): soft_flux(s, a, b) has the bits of the
-// hardware's RN(s * RN(b - a)) for every operand triple it covers, and pack undoes unpack, over
+// hardware's RN(s * RN(b - a)) for every operand triple it covers, soft_sub those of RN(b - a), and pack undoes unpack, over
 // random bit patterns, values of near and far exponents, neighbours a few ulps apart, sparse and
 // dense significands (ties), subnormals, huge values and specials.  Prints "cases N", "covered N"
 // and "bad N"; for ordinary values (exponents within +-60) "uncovered" must be 0.
@@ -53,11 +53,14 @@ int main(int argc, char** argv) {
     const double a = draw((int)(rnd() % 7), 1.0), b = draw((int)(rnd() % 8), a), s = draw((int)(rnd() % 7), 1.0);
     const softfp::SoftVal A = softfp::unpack(a), B = softfp::unpack(b);
     if (bits(softfp::pack(A)) != bits(a)) ++bad;
-    bool ok;
+    bool ok, okd;
+    const double diff = softfp::soft_sub(A, B, okd);
+    volatile double wantd = b - a;
+    if (okd && bits(diff) != bits(wantd)) ++bad;
     const double got = softfp::soft_flux(s, A, B, ok);
     auto ordinary = [](double v) { return v == 0.0 ? !std::signbit(v) : (std::fabs(v) > 1e-18 && std::fabs(v) < 1e18); };
     if (!ok) {
-      if (ordinary(a) && ordinary(b) && ordinary(s) && s != 0.0) ++uncovered;
+      if (ordinary(a) && ordinary(b) && ((ordinary(s) && s != 0.0) || !okd)) ++uncovered;
       continue;
     }
     ++covered;
