@@ -20,9 +20,9 @@
 //             free slot of its cell's slice, the particles taken in block order so that a warp's
 //             stores land in nearby slices (random particle order scatters them over the list:
 //             8.2 ms against 4.2 for 16.8 M particles on 256^3);
-//   4. fold   each window cell sorts its slice by particle index (an insertion sort: slots are
-//             taken in nearly increasing index order) and sums it from +0 in that order; a cell
-//             with no entry gets +0 (the reference's `dest <<= 0` before it adds).
+//   4. fold   the entries of each window cell's slice are ranked by particle index and summed from
+//             +0 in that order; a cell with no entry gets +0 (the reference's `dest <<= 0` before it
+//             adds).
 // CellToParticle and the fill spread a warp's (particle, cell) pairs evenly over its lanes, so
 // box sizes that differ between particles cost no divergence.  The floating-point work stays
 // on the FP64 pipe where the reference's bits require it (products, the weights' quotients,
@@ -125,12 +125,22 @@ __device__ __forceinline__ void make_axis(Axis& ax, double pos, double size, con
   ax.hi = (int)hi;
 }
 
+// Low and high coordinate of window cell i along one axis.
+struct __align__(16) CellFaces {
+  double cm, cp;
+};
+__device__ __forceinline__ CellFaces cell_faces(const PGeom& g, int a, int i) {
+  CellFaces f;
+  f.cm = __dadd_rn(g.face[a], __dmul_rn(fixmath::i32_to_f64(i), g.d[a]));
+  f.cp = __dadd_rn(f.cm, g.d[a]);
+  return f;
+}
+
 // Overlap of the particle with window cell i along one axis (1 when the axis is off).
 __device__ __forceinline__ double axis_cont(const Axis& ax, const PGeom& g, int a, int i) {
   if (!g.on[a]) return 1.0;
-  const double cm = __dadd_rn(g.face[a], __dmul_rn(fixmath::i32_to_f64(i), g.d[a]));
-  const double cp = __dadd_rn(cm, g.d[a]);
-  return __dsub_rn(dmin(cp, ax.phi), dmax(cm, ax.plo));
+  const CellFaces f = cell_faces(g, a, i);
+  return __dsub_rn(dmin(f.cp, ax.phi), dmax(f.cm, ax.plo));
 }
 
 // One (particle, value) entry of a cell's slice: 16 bytes, written with one store.
@@ -152,6 +162,11 @@ struct Box {
   __device__ __forceinline__ int count(int k) const { return a[k].hi > a[k].lo ? a[k].hi - a[k].lo : 0; }
 };
 
+__device__ __forceinline__ double box_volume(const PGeom& g, double size) {
+  const double two_rp = __dmul_rn(2.0, __dmul_rn(size, 0.5));
+  return __dmul_rn(__dmul_rn(g.on[0] ? two_rp : 1.0, g.on[1] ? two_rp : 1.0), g.on[2] ? two_rp : 1.0);
+}
+
 __device__ __forceinline__ void make_box(Box& b, const PGeom& g, const double* __restrict__ px,
                                          const double* __restrict__ py, const double* __restrict__ pz,
                                          const double* __restrict__ psize, long p) {
@@ -159,8 +174,7 @@ __device__ __forceinline__ void make_box(Box& b, const PGeom& g, const double* _
   make_axis(b.a[0], g.on[0] ? px[p] : 0.0, size, g, 0);
   make_axis(b.a[1], g.on[1] ? py[p] : 0.0, size, g, 1);
   make_axis(b.a[2], g.on[2] ? pz[p] : 0.0, size, g, 2);
-  const double two_rp = __dmul_rn(2.0, __dmul_rn(size, 0.5));
-  b.pvol = __dmul_rn(__dmul_rn(g.on[0] ? two_rp : 1.0, g.on[1] ? two_rp : 1.0), g.on[2] ? two_rp : 1.0);
+  b.pvol = box_volume(g, size);
 }
 
 using fixmath::div_by;
@@ -186,9 +200,9 @@ __device__ __forceinline__ long win_flat(const PGeom& g, int i, int j, int k) {
 // particle, over its lanes 32 at a time, so every lane does the same work per pair whatever the
 // box sizes.  For CellToParticle the owner lane then adds its pairs' products in that order.
 constexpr int PB = 4;
-constexpr int PWARPS = 8;  // warps per block
 constexpr int PCAP = 512;  // CellToParticle: products held per warp before the owners add them
 enum { PM_C2P = 0, PM_FILL = 2 };
+constexpr int PWARPS = 8;  // warps per block
 
 template <int MODE>
 struct WarpShared {
@@ -205,7 +219,7 @@ struct WarpShared {
 
 // One particle by its own lane, in the reference's loop order (boxes wider than PB cells).
 template <int MODE>
-__device__ __noinline__ double serial_particle(const PGeom& g, const double* __restrict__ px,
+__device__ __forceinline__ double serial_particle(const PGeom& g, const double* __restrict__ px,
                                                const double* __restrict__ py, const double* __restrict__ pz,
                                                const double* __restrict__ psize, long p,
                                                const double* __restrict__ cell, const double* __restrict__ src,
@@ -236,14 +250,33 @@ __device__ __noinline__ double serial_particle(const PGeom& g, const double* __r
   return acc;
 }
 
+// tab: the block's shared memory holds the faces of every window cell of each axis (3 FP64
+// operations per cell once, instead of once per particle and cell of its box; the window's edges
+// add up to PTAB cells or fewer).  The FP64 pipe bounds both modes (82 % busy in the gather): 2 M
+// particles, 18.8 M pairs: gather 731 -> 566 us, fill 617 -> 430 (506 with two blocks per SM; the
+// gather's products leave room for two).
+constexpr int PTAB = 1024;
+
 template <int MODE>
-__global__ void __launch_bounds__(PWARPS * 32, 2) particles_kernel(
-    PGeom g, const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
+__host__ __device__ constexpr size_t faces_offset() {  // the faces follow the warps' parts
+  return (PWARPS * sizeof(WarpShared<MODE>) + 15) / 16 * 16;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(PWARPS * 32, MODE == PM_C2P ? 2 : 3) particles_kernel(
+    const __grid_constant__ PGeom g, const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
     const double* __restrict__ psize, long np, const double* __restrict__ cell, double* __restrict__ dest,
     const double* __restrict__ src, const int* __restrict__ off, int* __restrict__ cnt, Entry* __restrict__ ent,
-    const int* __restrict__ order) {
+    const int* __restrict__ order, bool tab) {
   extern __shared__ __align__(16) unsigned char particle_smem[];
   WarpShared<MODE>* smem = reinterpret_cast<WarpShared<MODE>*>(particle_smem);
+  CellFaces* faces = reinterpret_cast<CellFaces*>(particle_smem + faces_offset<MODE>());
+    if (tab) {
+    const int n0 = g.nmax[0], n1 = n0 + g.nmax[1], n2 = n1 + g.nmax[2];
+    for (int i = threadIdx.x; i < n2; i += PWARPS * 32)
+      faces[i] = i < n0 ? cell_faces(g, 0, i) : (i < n1 ? cell_faces(g, 1, i - n0) : cell_faces(g, 2, i - n1));
+    __syncthreads();
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpShared<MODE>& sm = smem[warp];
   for (long base = ((long)blockIdx.x * PWARPS + warp) * 32; base < np; base += (long)gridDim.x * PWARPS * 32) {
@@ -253,25 +286,39 @@ __global__ void __launch_bounds__(PWARPS * 32, 2) particles_kernel(
     int npairs = 0;
     bool big = false;
     if (base + lane < np) {
-      Box b;
-      make_box(b, g, px, py, pz, psize, p);
-      const int n0 = b.count(0), n1 = b.count(1), n2 = b.count(2);
+      // one axis after the other: its box and, at once, the overlaps with its first PB cells
+      const double size = psize[p];
+      const double* pos[3] = {px, py, pz};
+      int n[3], base = 0;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        Axis ax;
+        make_axis(ax, g.on[a] ? pos[a][p] : 0.0, size, g, a);
+        n[a] = ax.hi > ax.lo ? ax.hi - ax.lo : 0;
+        sm.lo[a][lane] = ax.lo;
+        const int m = n[a] < PB ? n[a] : PB;
+        for (int t = 0; t < m; ++t) {
+          double c = 1.0;
+          if (g.on[a]) {
+            const CellFaces f = tab ? faces[base + ax.lo + t] : cell_faces(g, a, ax.lo + t);
+            c = __dsub_rn(dmin(f.cp, ax.phi), dmax(f.cm, ax.plo));
+          }
+          sm.cont[a][t][lane] = c;
+        }
+        base += g.nmax[a];
+      }
+      const int n0 = n[0], n1 = n[1], n2 = n[2];
       const long cells = (long)n0 * n1 * n2;
       big = cells > 0 && (n0 > PB || n1 > PB || n2 > PB);
       if (cells > 0 && !big) {
         npairs = (int)cells;
         sm.n[0][lane] = n0;
         sm.n[1][lane] = n1;
-        sm.lo[0][lane] = b.a[0].lo;
-        sm.lo[1][lane] = b.a[1].lo;
-        sm.lo[2][lane] = b.a[2].lo;
         sm.mxy[lane] = 65536u / (unsigned)(n0 * n1) + 1u;
         sm.mx[lane] = 65536u / (unsigned)n0 + 1u;
-        sm.pvol[lane] = b.pvol;
-        sm.rcp[lane] = __drcp_rn(b.pvol);
-        for (int t = 0; t < n0; ++t) sm.cont[0][t][lane] = axis_cont(b.a[0], g, 0, b.a[0].lo + t);
-        for (int t = 0; t < n1; ++t) sm.cont[1][t][lane] = axis_cont(b.a[1], g, 1, b.a[1].lo + t);
-        for (int t = 0; t < n2; ++t) sm.cont[2][t][lane] = axis_cont(b.a[2], g, 2, b.a[2].lo + t);
+        const double pvol = box_volume(g, size);
+        sm.pvol[lane] = pvol;
+        sm.rcp[lane] = __drcp_rn(pvol);
         if (MODE == PM_FILL) {
           sm.val[lane] = src[p];
           sm.pid[lane] = p;
@@ -375,11 +422,14 @@ __global__ void __launch_bounds__(256) p2c_order_kernel(const int* __restrict__ 
 }
 
 // Fold of ParticleToCell: a warp takes 32 consecutive window cells, whose slices form one
-// contiguous run of the entry list.  It stages the run in shared memory with coalesced loads,
-// in groups of consecutive lanes whose slices fit in FCAP entries, and each lane of a group
-// sorts its cell's slice by particle index (an insertion sort: the slots were taken in nearly
-// increasing order) and adds it from +0 in that order.  A single slice longer than FCAP is
-// sorted and added where it lies, in global memory.
+// contiguous run of the entry list, in groups of consecutive lanes whose slices fit in FCAP entries.
+// Each entry's place within its slice is the number of smaller particle indices there (an entry per
+// lane, the slice's indices read from shared memory: no lane waits for another's comparisons), the
+// values go to their places in shared memory and each lane adds its cell's from +0 in that order.
+// A single slice longer than FCAP is sorted and added where it lies, in global memory.
+// What bounds it: issue, about 20 comparisons per entry at 18 entries a cell.  2 M particles, 18.8 M
+// entries: 717 us with an insertion sort per lane (the slots are in nearly random order, since the
+// fill takes particles in block order), 217 us; FCAP 320, 640, 1024: 250, 317, 285 us.
 constexpr int FCAP = 512;
 constexpr int FWARPS = 4;
 
@@ -396,10 +446,18 @@ __device__ __forceinline__ void fold_slice(Entry* e, int n, double& acc) {
   for (int s = 0; s < n; ++s) acc = __dadd_rn(acc, e[s].val);
 }
 
+struct FoldShared {
+  double val[FCAP];
+  int pid[FCAP];       // particle indices are below 2^31
+  unsigned char cell[FCAP];  // the entry's cell (lane)
+  int off[33];         // slices of the lanes' cells in the staged run
+};
+
 __global__ void __launch_bounds__(FWARPS * 32) p2c_fold_kernel(PGeom g, long ncell, const int* __restrict__ off,
                                                                Entry* __restrict__ ent, double* __restrict__ dest) {
-  __shared__ Entry stage[FWARPS][FCAP];
+  extern __shared__ __align__(16) unsigned char fold_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  FoldShared& sm = reinterpret_cast<FoldShared*>(fold_smem)[warp];
   const long nxy = (long)g.nmax[0] * g.nmax[1];
   for (long c0 = ((long)blockIdx.x * FWARPS + warp) * 32; c0 < ncell; c0 += (long)gridDim.x * FWARPS * 32) {
     const long c = c0 + lane;
@@ -417,18 +475,27 @@ __global__ void __launch_bounds__(FWARPS * 32) p2c_fold_kernel(PGeom g, long nce
       if (!fits) {
         if (lane == first) fold_slice(ent + b, e - b, acc);  // one slice longer than FCAP
       } else {
-        const int r1 = __shfl_sync(0xffffffffu, e, last);
-        for (int t = r0 + lane; t < r1; t += 128) {
-          Entry v[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (t + 32 * u < r1) v[u] = ent[t + 32 * u];
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (t + 32 * u < r1) stage[warp][t + 32 * u - r0] = v[u];
+        const int n = __shfl_sync(0xffffffffu, e, last) - r0;
+        if (mine) {
+          sm.off[lane] = b - r0;
+          if (lane == last) sm.off[lane + 1] = e - r0;
+          for (int t = b - r0; t < e - r0; ++t) sm.cell[t] = (unsigned char)lane;
+        }
+        // stage the indices; this lane's entries' values stay in registers, 4 at a time, until
+        // every index is there
+        for (int t = lane; t < n; t += 32) sm.pid[t] = (int)ent[r0 + t].pid;
+        __syncwarp();
+        for (int t = lane; t < n; t += 32) {
+          const double v = ent[r0 + t].val;
+          const int me = sm.pid[t], cl = sm.cell[t], f = sm.off[cl], m = sm.off[cl + 1] - f;
+          int rank = 0;
+#pragma unroll 4
+          for (int q = 0; q < m; ++q) rank += sm.pid[f + q] < me ? 1 : 0;
+          sm.val[f + rank] = v;
         }
         __syncwarp();
-        if (mine) fold_slice(&stage[warp][b - r0], e - b, acc);
+        if (mine)
+          for (int t = b - r0; t < e - r0; ++t) acc = __dadd_rn(acc, sm.val[t]);
         __syncwarp();
       }
       first = last + 1;
@@ -555,21 +622,33 @@ int particle_geom(const nebo_particle_mesh* mesh, const nebo_field* cell, const 
   return NEBO_OK;
 }
 
-int particle_blocks(long np, int per_sm = 6) {
-  long b = (np + PWARPS * 32 - 1) / (PWARPS * 32);
+// Whether the faces of all window cells go into shared memory, and the bytes a block takes.
+bool use_faces(const PGeom& g) { return (long)g.nmax[0] + g.nmax[1] + g.nmax[2] <= PTAB; }
+template <int MODE>
+size_t particle_smem_bytes(const PGeom& g) {
+  const size_t faces = use_faces(g) ? ((size_t)g.nmax[0] + g.nmax[1] + g.nmax[2]) * sizeof(CellFaces) : 0;
+  return faces_offset<MODE>() + faces;
+}
+
+int particle_blocks(long np, int threads, int per_sm) {
+  long b = (np + threads - 1) / threads;
   const long cap = (long)num_sms() * per_sm;
   if (b > cap) b = cap;
   return (int)(b < 1 ? 1 : b);
 }
 
-// CellToParticle's shared memory exceeds the 48 KB default; opt in once per device.
-int c2p_prepare() {
+// CellToParticle's and the fold's shared memory exceed the 48 KB default; opt in once per device.
+int particles_prepare(const char* who) {
   static std::atomic<unsigned long long> done{0};
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return cuda_fail(cudaGetLastError(), "nebo_cell_to_particle");
+  if (cudaGetDevice(&dev) != cudaSuccess) return cuda_fail(cudaGetLastError(), who);
   if (dev < 64 && (done.load() & (1ull << dev))) return NEBO_OK;
+  NEBO_CUDA_TRY(cudaFuncSetAttribute(p2c_fold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(FWARPS * sizeof(FoldShared))));
   NEBO_CUDA_TRY(cudaFuncSetAttribute(particles_kernel<PM_C2P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(PWARPS * sizeof(WarpShared<PM_C2P>))));
+                                     (int)(faces_offset<PM_C2P>() + PTAB * sizeof(CellFaces))));
+  NEBO_CUDA_TRY(cudaFuncSetAttribute(particles_kernel<PM_FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(faces_offset<PM_FILL>() + PTAB * sizeof(CellFaces))));
   if (dev < 64) done.fetch_or(1ull << dev);
   return NEBO_OK;
 }
@@ -589,12 +668,12 @@ extern "C" int nebo_cell_to_particle(const nebo_particle_mesh* mesh, const doubl
   if (nparticles == 0) return NEBO_OK;
   if (!psize || !dest) return fail(NEBO_ERR_INVALID, "Nebo error in %s: null particle size or destination", who);
   cudaStream_t s = (cudaStream_t)stream;
-  if (int rc = c2p_prepare()) return rc;
+  if (int rc = particles_prepare("nebo_cell_to_particle")) return rc;
   {
     LaunchScope ls("cell_to_particle", s);
-    particles_kernel<PM_C2P><<<particle_blocks(nparticles), PWARPS * 32, PWARPS * sizeof(WarpShared<PM_C2P>), s>>>(
+    particles_kernel<PM_C2P><<<particle_blocks(nparticles, PWARPS * 32, 6), PWARPS * 32, particle_smem_bytes<PM_C2P>(g), s>>>(
         g, px, py, pz, psize, (long)nparticles, static_cast<const double*>(cell->data), dest, nullptr, nullptr,
-        nullptr, nullptr, nullptr);
+        nullptr, nullptr, nullptr, use_faces(g));
   }
   NEBO_LAUNCH_CHECK("nebo_cell_to_particle");
   return NEBO_OK;
@@ -615,6 +694,7 @@ extern "C" int nebo_particle_to_cell(const nebo_particle_mesh* mesh, const doubl
   if (ncell <= 0) return NEBO_OK;
   if (ncell >= (1L << 31) - 1) return fail(NEBO_ERR_UNSUPPORTED, "Nebo error in %s: window above 2^31-2 cells", who);
   cudaStream_t s = (cudaStream_t)stream;
+  if (int rc = particles_prepare("nebo_particle_to_cell")) return rc;
   // the scan runs over ncell + 1 counters (the last one stays 0), so off[ncell] is the total
   const long nscan = ncell + 1;
   const long ntile = (nscan + SCAN_TILE - 1) / SCAN_TILE;
@@ -657,7 +737,7 @@ extern "C" int nebo_particle_to_cell(const nebo_particle_mesh* mesh, const doubl
   if (nparticles > 0) {
     {
       LaunchScope ls("particle_to_cell_count", s);
-      p2c_count_kernel<<<particle_blocks(nparticles, 16), 256, 0, s>>>(g, px, py, pz, psize, (long)nparticles, cnt,
+      p2c_count_kernel<<<particle_blocks(nparticles, 256, 16), 256, 0, s>>>(g, px, py, pz, psize, (long)nparticles, cnt,
                                                                    total, key, hist, kbx, kby, nkey);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) {
@@ -698,7 +778,7 @@ extern "C" int nebo_particle_to_cell(const nebo_particle_mesh* mesh, const doubl
       scan_tile_sums_kernel<<<(unsigned)nktile, SCAN_THREADS, 0, s>>>(hist, nkscan, bsum);
       scan_block_sums_kernel<<<1, SCAN_THREADS, 0, s>>>(bsum, (int)nktile, grand);
       scan_tile_apply_kernel<<<(unsigned)nktile, SCAN_THREADS, 0, s>>>(hist, nkscan, bsum, hpos);
-      p2c_order_kernel<<<particle_blocks(nparticles, 16), 256, 0, s>>>(key, (long)nparticles, hpos, order);
+      p2c_order_kernel<<<particle_blocks(nparticles, 256, 16), 256, 0, s>>>(key, (long)nparticles, hpos, order);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) {
       rc = cuda_fail(e, "nebo_particle_to_cell order");
@@ -710,8 +790,8 @@ extern "C" int nebo_particle_to_cell(const nebo_particle_mesh* mesh, const doubl
     }
     {
       LaunchScope ls("particle_to_cell_fill", s);
-      particles_kernel<PM_FILL><<<particle_blocks(nparticles), PWARPS * 32, PWARPS * sizeof(WarpShared<PM_FILL>), s>>>(
-          g, px, py, pz, psize, (long)nparticles, nullptr, nullptr, src, off, cnt, ent, order);
+      particles_kernel<PM_FILL><<<particle_blocks(nparticles, PWARPS * 32, 6), PWARPS * 32, particle_smem_bytes<PM_FILL>(g), s>>>(
+          g, px, py, pz, psize, (long)nparticles, nullptr, nullptr, src, off, cnt, ent, order, use_faces(g));
     }
     if ((e = cudaGetLastError()) != cudaSuccess) {
       rc = cuda_fail(e, "nebo_particle_to_cell fill");
@@ -723,7 +803,7 @@ extern "C" int nebo_particle_to_cell(const nebo_particle_mesh* mesh, const doubl
     const long cap = (long)num_sms() * 8;
     if (nb > cap) nb = cap;
     LaunchScope ls("particle_to_cell_fold", s);
-    p2c_fold_kernel<<<(unsigned)nb, FWARPS * 32, 0, s>>>(g, ncell, off, ent, static_cast<double*>(cell->data));
+    p2c_fold_kernel<<<(unsigned)nb, FWARPS * 32, FWARPS * sizeof(FoldShared), s>>>(g, ncell, off, ent, static_cast<double*>(cell->data));
   }
   if ((e = cudaGetLastError()) != cudaSuccess) rc = cuda_fail(e, "nebo_particle_to_cell fold");
 done:
