@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
     sm.ay[buf][ty][tx] = day;
     extra(buf);
   };
+  step_begin();
   double tn, an, ac, tn2, an2, dazl, dtzl, dazh, dtzh;
   SoftVal X, Y;  // T and A of plane z + 1
   {
@@ -319,6 +320,7 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
         stage(buf, 1, hi, __ldg(Ain + (long)sz * (z + 2) + ih));
       }
     }
+    if (!more) step_end();
     store(z, v, gn);
     if (!more) break;
     ac = an;
@@ -419,7 +421,7 @@ int adjoint_step_lf(const nebo_field* Tk, const nebo_field* Ain, const nebo_fiel
         const int zchunk =
             wave_zchunk((long)gxb * gyb, (long)num_sms() * blocks_per_sm(kern, BX * BY, cache), n[2], 2, 4, 1);
         LaunchScope ls("heat_adjoint_step", s);
-        kern<<<dim3(gxb, gyb, (n[2] + zchunk - 1) / zchunk), dim3(BX, BY), 0, s>>>(
+        launch_step_kernel(kern, dim3(gxb, gyb, (n[2] + zchunk - 1) / zchunk), dim3(BX, BY), 0, s,
             vt.base, va.base, vo.base, lfx, lfy, lfz, vg.base, vt.sy, (int)vt.sz, n[0], n[1], n[2], zchunk, 0.5 * dt);
       };
       if (exact)

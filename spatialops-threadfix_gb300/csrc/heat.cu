@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(BX* BY) heat_step_kernel(const T* __restrict__
   const int xc = min(x, nx), yc = min(y, ny);
   auto at = [&](int i, int j, int k) { return (long)i + (long)sy * j + sz * k; };
 
+  step_begin();
   T tc = __ldg(tin + at(xc, yc, z0));
   T lc = __ldg(lam + at(xc, yc, z0));
   T fzlo = face_flux<T, A, MODE>(__ldg(lam + at(xc, yc, z0 - 1)), lc, __ldg(tin + at(xc, yc, z0 - 1)), tc, p.c0[2],
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(BX* BY) heat_step_kernel(const T* __restrict__
       }
     }
     __syncthreads();
+    if (z + 1 == z1) step_end();
     if (active) {
       const T fxhi = sfx[buf][ty][tx + 1];
       const T fyhi = sfy[buf][ty + 1][tx];
@@ -1046,6 +1048,7 @@ __global__ void __launch_bounds__(BP_THREADS, 3) heat_step_f32_bulk2_kernel(cons
   const int tid = threadIdx.x;
   const int y0 = blockIdx.x * BK_RY;
   const int z0 = blockIdx.y * zchunk, z1 = min(z0 + zchunk, nz);
+  step_begin();
   if (tid == 0) {
     for (int st = 0; st < BK_NS; ++st) mbar_init(bar0 + 8 * st, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1089,7 +1092,8 @@ __global__ void __launch_bounds__(BP_THREADS, 3) heat_step_f32_bulk2_kernel(cons
 #pragma unroll 1
   for (int z = z0; z < z1; ++z) {
     const int q = z - z0 + 1;  // centre plane
-    __syncthreads();           // plane q-1's stage is no longer read
+    if (z + 1 == z1) step_end();
+    __syncthreads();  // plane q-1's stage is no longer read
     if (tid == 0) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       issue(q - 1 + BK_NS);
@@ -1170,6 +1174,7 @@ __global__ void __maxnreg__(40)
   const uint32_t bar0 = s0 + (uint32_t)NS * 2u * fb;
   const int x = threadIdx.x, y0 = blockIdx.x * SR;
   const int z0 = blockIdx.y * zchunk, z1 = min(z0 + zchunk, nz);
+  step_begin();
   if (x == 0) {
     for (int st = 0; st < NS; ++st) mbar_init(bar0 + 8 * st, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1309,11 +1314,11 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
     dim3 grid(gxb, gyb, (n[2] + zchunk - 1) / zchunk), block(BX, BY);
     LaunchScope ls("heat_step_f64", s);
     if (unit)
-      heat_step_kernel<double, ExactD, MODE_UNIT><<<grid, block, 0, s>>>(vin.base, vout.base, vl.base, vin.sy, vin.sz,
-                                                                         n[0], n[1], n[2], zchunk, p);
+      launch_step_kernel(heat_step_kernel<double, ExactD, MODE_UNIT>, grid, block, 0, s, vin.base, vout.base, vl.base,
+                         vin.sy, vin.sz, n[0], n[1], n[2], zchunk, p);
     else
-      heat_step_kernel<double, ExactD, MODE_REFERENCE><<<grid, block, 0, s>>>(vin.base, vout.base, vl.base, vin.sy,
-                                                                              vin.sz, n[0], n[1], n[2], zchunk, p);
+      launch_step_kernel(heat_step_kernel<double, ExactD, MODE_REFERENCE>, grid, block, 0, s, vin.base, vout.base,
+                         vl.base, vin.sy, vin.sz, n[0], n[1], n[2], zchunk, p);
   } else {
     // bulk-copied slabs in packed pairs: rows of 16-byte aligned windows with an even pitch, 8 rows
     // per block.  Its 128 pair columns want wide rows: against the scalar slab kernel below it takes
@@ -1336,9 +1341,8 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
       const int ch = max(1, min(num_sms() * bps / yb, n[2]));
       const int zc = (n[2] + ch - 1) / ch;
       LaunchScope ls("heat_step_f32", s);
-      kern<<<dim3(yb, (n[2] + zc - 1) / zc), BP_THREADS, bk_smem, s>>>(
-          (const float*)Tf->data, vout.base, (const float*)Lf->data, gx, vin.sz, n[0], n[1], n[2], zc, p.w[0], p.w[1],
-          p.w[2]);
+      launch_step_kernel(kern, dim3(yb, (n[2] + zc - 1) / zc), dim3(BP_THREADS), bk_smem, s, (const float*)Tf->data,
+                         vout.base, (const float*)Lf->data, gx, vin.sz, n[0], n[1], n[2], zc, p.w[0], p.w[1], p.w[2]);
       NEBO_LAUNCH_CHECK("nebo_heat_step");
       return NEBO_OK;
     }
@@ -1357,9 +1361,8 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
       const int zc = (n[2] + ch - 1) / ch;
       const long total = (long)gx * gy * Tf->glob[2];
       LaunchScope ls("heat_step_f32", s);
-      kern<<<dim3(yb, (n[2] + zc - 1) / zc), bx, smem, s>>>((const float*)Tf->data, vout.base, (const float*)Lf->data,
-                                                            total, gx, vin.sz, n[0], n[1], n[2], zc, p.w[0], p.w[1],
-                                                            p.w[2]);
+      launch_step_kernel(kern, dim3(yb, (n[2] + zc - 1) / zc), dim3(bx), smem, s, (const float*)Tf->data, vout.base,
+                         (const float*)Lf->data, total, gx, vin.sz, n[0], n[1], n[2], zc, p.w[0], p.w[1], p.w[2]);
       NEBO_LAUNCH_CHECK("nebo_heat_step");
       return NEBO_OK;
     }
@@ -1542,11 +1545,11 @@ int heat_step_faces(const nebo_field* Tf, const nebo_field* Tof, const double* c
   const dim3 grid(gxb, gyb, (n[2] + zchunk - 1) / zchunk), block(HS_X, HS_Y);
   LaunchScope ls("heat_step_f64", s);
   if (unit)
-    heat_soft_kernel<true><<<grid, block, 0, s>>>(vin.base, vout.base, lf[0], lf[1], lf[2], vin.sy, (int)vin.sz, n[0],
-                                                  n[1], n[2], zchunk, p);
+    launch_step_kernel(heat_soft_kernel<true>, grid, block, 0, s, vin.base, vout.base, lf[0], lf[1], lf[2], vin.sy,
+                       (int)vin.sz, n[0], n[1], n[2], zchunk, p);
   else
-    heat_soft_kernel<false><<<grid, block, 0, s>>>(vin.base, vout.base, lf[0], lf[1], lf[2], vin.sy, (int)vin.sz, n[0],
-                                                   n[1], n[2], zchunk, p);
+    launch_step_kernel(heat_soft_kernel<false>, grid, block, 0, s, vin.base, vout.base, lf[0], lf[1], lf[2], vin.sy,
+                       (int)vin.sz, n[0], n[1], n[2], zchunk, p);
   NEBO_LAUNCH_CHECK("nebo_heat_run");
   return NEBO_OK;
 }

@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(HS_X* HS_Y, UNIT ? 4 : 3) heat_soft_kernel(
     }
   };
 
+  step_begin();
   // plane z0: staged, its low z face and its other faces
   double tc, tn, tn2, hn = 0.0, fzlo, fzhi, fx, fy;
   SoftVal X, Z;  // of plane z + 1 (in general spacing scaled for its x and z faces)
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(HS_X* HS_Y, UNIT ? 4 : 3) heat_soft_kernel(
       c = __dsub_rn(__dmul_rn(fzhi, p.c1[2]), __dmul_rn(fzlo, p.c1[2]));
     }
     if (z + 1 >= z1) {
+      step_end();
       store(z, __dadd_rn(tc, __dmul_rn(p.hdt, __dadd_rn(__dadd_rn(a, b), c))));
       break;
     }

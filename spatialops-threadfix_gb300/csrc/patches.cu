@@ -336,6 +336,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) patches_soft_kernel(const Patch
                                                                      const double* __restrict__ src,
                                                                      double* __restrict__ dst) {
   __shared__ PatchSoftAny sm;
+  step_begin();
   for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
     const WorkItem it = items[w];
     const PatchDev P = patches[it.patch];
@@ -347,6 +348,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4) patches_soft_kernel(const Patch
       patch_soft_item<6>(sm.s6, P, it, src, dst);
     __syncthreads();  // the staged planes and faces are reused by the next item
   }
+  step_end();
 }
 
 // FP32 mode shares the ring machinery of the FP32 heat step: plane p (z0-1 <= p <= z1) lives in
@@ -561,6 +563,7 @@ __global__ void __launch_bounds__(PT_THREADS) patches_f32_bulk_kernel(const Patc
   const uint32_t bar0 = ring0 + (uint32_t)(PB_NS * stage_floats) * 4u;
   const int tid = threadIdx.x;
   bool ok = true;
+  step_begin();
   for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
     const WorkItem it = items[w];
     const PatchDev P = patches[it.patch];
@@ -642,6 +645,7 @@ __global__ void __launch_bounds__(PT_THREADS) patches_f32_bulk_kernel(const Patc
     if (tid == 0)
       for (int st = 0; st < PB_NS; ++st) mbar_inval(bar0 + 8 * st);
   }
+  step_end();
   if (!ok) atomicAdd(&g_patch_bulk_timeouts, 1u);
 }
 
@@ -826,12 +830,12 @@ int launch_step(const PatchSet& ps, const WorkItem* items, int nitems, int parit
                                                                (const double*)ps.arena[parity],
                                                                (double*)ps.arena[parity ^ 1]);
   else if (ps.dtype == NEBO_F64)
-    patches_soft_kernel<<<grid, PT_THREADS, 0, s>>>(ps.d_patches, items, nitems, (const double*)ps.arena[parity],
-                                                    (double*)ps.arena[parity ^ 1]);
+    launch_step_kernel(patches_soft_kernel, dim3(grid), dim3(PT_THREADS), 0, s, ps.d_patches, items, nitems,
+                       (const double*)ps.arena[parity], (double*)ps.arena[parity ^ 1]);
   else if (ps.dtype == NEBO_F32 && ps.bulk32)
-    patches_f32_bulk_kernel<<<std::min(nitems, ps.grid32), PT_THREADS,
-                              (size_t)PB_NS * ps.stage32 * sizeof(float) + PB_NS * sizeof(uint64_t), s>>>(
-        ps.d_patches, items, nitems, ps.arena32[parity], ps.arena32[parity ^ 1], ps.stage32);
+    launch_step_kernel(patches_f32_bulk_kernel, dim3(std::min(nitems, ps.grid32)), dim3(PT_THREADS),
+                       (size_t)PB_NS * ps.stage32 * sizeof(float) + PB_NS * sizeof(uint64_t), s, ps.d_patches, items,
+                       nitems, ps.arena32[parity], ps.arena32[parity ^ 1], ps.stage32);
   else if (ps.dtype == NEBO_F32)
     patches_f32_strip_kernel<<<std::min(nitems, ps.grid32), PT_THREADS, 0, s>>>(ps.d_patches, items, nitems,
                                                                                ps.arena32[parity],

@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
   const bool xface = (ty == 0 && y0 + TY <= n && x <= n) || (ty == 1 && tx < TY && x0 + TX <= n && y0 + tx < n);
   const long c0 = (long)xc + (long)sy * yc;
   const long ce = ty == 0 ? (long)xc + (long)sy * (y0 + TY) : (long)(x0 + TX) + (long)sy * (y0 + tx);
+  step_begin();
   long c = c0 + sz * z0;
   double pm1 = __ldg(a.phi + c - sz), p0 = __ldg(a.phi + c), p1 = __ldg(a.phi + c + sz);
   double fzlo = flux(coef(kfz, c, sz), __ldg(a.w + c), __ldg(a.phi + c - 2 * sz), pm1, p0, p1);
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
     const double fzhi = flux(coef(kfz, c + sz, sz), __ldg(a.w + c + sz), pm1, p0, p1, p2);
     const double dz = fzhi - fzlo;
     __syncthreads();
+    if (z + 1 == z1) step_end();
     if (active) {
       const double rhs = ((sfx[buf][ty][tx + 1] - fx) + (sfy[buf][ty + 1][tx] - fy)) + dz;
       double r = fma(a.dt, rhs, p0);  // FP64 stages advance from the state they read
@@ -535,6 +537,7 @@ __global__ void __launch_bounds__(PTX* TY) transport_stage_f32_pair_kernel(TrArg
     }
   };
   bool ok = true;
+  step_begin();
   if constexpr (TMA) {
     if (tid == 0) {
       for (int st = 0; st < SNS; ++st) mbar_init(bar0 + 8u * st, 1);
@@ -580,6 +583,7 @@ __global__ void __launch_bounds__(PTX* TY) transport_stage_f32_pair_kernel(TrArg
   for (int z = z0; z < z1; ++z) {
     const int i = z - z0;
     const Col nxt = load_col(min(z + 1, n));  // plane n is a ghost plane: valid memory
+    if (z + 1 == z1) step_end();
     if constexpr (TMA) {
       // planes z and z+1 were waited for as the newest planes of the two previous iterations
       if (i == 0) ok &= mbar_wait(bar0, 0) & mbar_wait(bar0 + 8u, 0);
@@ -670,7 +674,8 @@ int transport_launch_f64(const TrArgs<double>& a, const double* const kf[3], dou
     const int zchunk =
         wave_zchunk((long)gxb * gyb, (long)num_sms() * blocks_per_sm(kern, TX * TY, cache), n, 2 * G, 8, 1);
     LaunchScope ls("transport_stage_f64", s);
-    kern<<<dim3(gxb, gyb, (n + zchunk - 1) / zchunk), dim3(TX, TY), 0, s>>>(a, kf[0], kf[1], kf[2], kc, zchunk);
+    launch_step_kernel(kern, dim3(gxb, gyb, (n + zchunk - 1) / zchunk), dim3(TX, TY), 0, s, a, kf[0], kf[1], kf[2],
+                       kc, zchunk);
   };
   if (kf[0]) {
     if (second) go(transport_stage_f64_kernel<true, true>); else go(transport_stage_f64_kernel<false, true>);
@@ -749,18 +754,18 @@ int transport_launch(TrArgs<float> a, bool second, cudaStream_t s, const TrMaps*
   {
     if (kind == 3) {
       if (second)
-        transport_stage_f32_pair_kernel<true, true><<<grid, dim3(PTX, TY), 0, s>>>(a, zchunk, *maps);
+        launch_step_kernel(transport_stage_f32_pair_kernel<true, true>, grid, dim3(PTX, TY), 0, s, a, zchunk, *maps);
       else
-        transport_stage_f32_pair_kernel<false, true><<<grid, dim3(PTX, TY), 0, s>>>(a, zchunk, *maps);
+        launch_step_kernel(transport_stage_f32_pair_kernel<false, true>, grid, dim3(PTX, TY), 0, s, a, zchunk, *maps);
       NEBO_LAUNCH_CHECK("nebo_transport_run");
       return NEBO_OK;
     }
     if (kind == 2) {
       const TrMaps none{};
       if (second)
-        transport_stage_f32_pair_kernel<true, false><<<grid, dim3(PTX, TY), 0, s>>>(a, zchunk, none);
+        launch_step_kernel(transport_stage_f32_pair_kernel<true, false>, grid, dim3(PTX, TY), 0, s, a, zchunk, none);
       else
-        transport_stage_f32_pair_kernel<false, false><<<grid, dim3(PTX, TY), 0, s>>>(a, zchunk, none);
+        launch_step_kernel(transport_stage_f32_pair_kernel<false, false>, grid, dim3(PTX, TY), 0, s, a, zchunk, none);
       NEBO_LAUNCH_CHECK("nebo_transport_run");
       return NEBO_OK;
     }
