@@ -184,35 +184,47 @@ __global__ void __launch_bounds__(PT_THREADS) patches_step_kernel(const PatchDev
 // update, arranged as in heat_soft.cuh: values are unpacked once and staged with their halo two
 // planes ahead, the update of plane z runs beside the integer fluxes of plane z + 1.  The same bits
 // as FP64 fluxes: 9 FP64 operations per cell instead of 13, which is what bounds the step (with the
-// lanes that a tile's ragged edge leaves idle).  128 patches of 16..96 cells an edge: 816 -> 612 us
-// per step; z chunks of 16 planes (32: 608, but 20 small patches 47 -> 58).
-template <int LX>
+// lanes that a tile's ragged edge leaves idle).  128 patches of 16..96 cells an edge: 816 -> 560 us
+// per step (612 with tiles of 16, 32 or 64 columns and z chunks of 16 planes).
+//
+// Tile shape: at most 2^log2tx columns (the autotuner's choice) and 256 cells, the patch's columns
+// and then its rows split evenly, so that few lanes idle whatever the patch's extents (the FP64
+// pipe's time goes by warps).  At most 64 rows: the tile's halo cells and faces have a thread each.
+__host__ __device__ __forceinline__ void tile_shape(int nx, int ny, int log2tx, int& TX, int& TY) {
+  const int lim = 1 << log2tx, kx = (nx + lim - 1) / lim;
+  TX = (nx + kx - 1) / kx;
+  const int most = PT_THREADS / TX < 64 ? PT_THREADS / TX : 64, ky = (ny + most - 1) / most;
+  TY = (ny + ky - 1) / ky;
+}
+constexpr int PSOFT_CELLS = 400;  // max (TX + 2)(TY + 2): 66 x 6
 struct PatchSoftShared {
-  static constexpr int TX = 1 << LX, TY = PT_THREADS >> LX, W = TX + 2;
-  long long m[2][(TY + 2) * W];
-  int e[2][(TY + 2) * W];
-  double fx[2][TY * (TX + 1)];
-  double fy[2][(TY + 1) * TX];
-};
-union PatchSoftAny {
-  PatchSoftShared<4> s4;
-  PatchSoftShared<5> s5;
-  PatchSoftShared<6> s6;
+  long long m[2][PSOFT_CELLS];
+  int e[2][PSOFT_CELLS];
+  double fx[2][PT_THREADS + 64];  // TY (TX + 1)
+  double fy[2][PT_THREADS + 64];  // (TY + 1) TX
+  int2 halo[PT_THREADS - 64];     // a halo cell's offset in a plane and staged index
+  PatchDev P;                     // the item at hand (its 64 registers are taken)
+  WorkItem it;
 };
 
-template <int LX>
-__device__ __forceinline__ void patch_soft_item(PatchSoftShared<LX>& sm, const PatchDev& P, const WorkItem& it,
-                                                const double* __restrict__ src, double* __restrict__ dst) {
-  constexpr int TX = 1 << LX, TY = PT_THREADS >> LX, W = TX + 2;
+__device__ __forceinline__ void patch_soft_item(PatchSoftShared& sm, const double* __restrict__ src,
+                                                double* __restrict__ dst) {
   using softfp::SoftVal;
-  const int tid = threadIdx.x, tx = tid & (TX - 1), ty = tid >> LX;
+  const PatchDev& P = sm.P;
+  const WorkItem& it = sm.it;
+  int TX, TY;
+  tile_shape(P.nx, P.ny, P.log2tx, TX, TY);
+  const int W = TX + 2, tid = threadIdx.x;
+  // threads beyond the tile repeat its first cell and store nothing
+  const bool in_tile = tid < TX * TY;
+  const int ty = in_tile ? tid / TX : 0, tx = in_tile ? tid - ty * TX : 0;
   const int nx = P.nx, ny = P.ny, nz = P.nz, sy = nx + 2, sz = (nx + 2) * (ny + 2);
   const double s = P.lam2, hdt = P.hdt;
   const double* tin = src + P.offset + 1 + sy + sz;  // interior (0, 0, 0)
   double* tout = dst + P.offset + 1 + sy + sz;
   const int x0 = it.x0, y0 = it.y0, z0 = it.z0, z1 = it.z1;
   const int ic = min(x0 + tx, nx) + sy * min(y0 + ty, ny);
-  const int si = (ty + 1) * W + tx + 1;
+  const int si = (ty + 1) * W + tx + 1, fi = ty * (TX + 1) + tx, gi = ty * TX + tx;
   auto hard = [&](SoftVal a, SoftVal b) { return __dmul_rn(s, __dsub_rn(softfp::pack(b), softfp::pack(a))); };
   auto stage = [&](int buf, int i, double t) {
     const SoftVal v = softfp::unpack(t);
@@ -226,19 +238,24 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared<LX>& sm, const P
     v.e = sm.e[buf][i];
     return v;
   };
-  // halo cells, from thread 64 on: columns x0 + TX and x0 - 1, rows y0 - 1 and y0 + TY (clamped into
-  // the window; a clamped cell feeds no active face)
+  // halo cells, from thread 64 on (2 (TX + TY) <= 192 of them): columns x0 + TX and x0 - 1, rows
+  // y0 - 1 and y0 + TY (clamped into the window; a clamped cell feeds no active face)
   const int h = tid - 64;
   const bool halo = h >= 0 && h < 2 * TY + 2 * TX;
-  int ih, hi;
-  if (h < 2 * TY) {
-    const int r = h & (TY - 1);
-    ih = (h < TY ? min(x0 + TX, nx) : x0 - 1) + sy * min(y0 + r, ny);
-    hi = (r + 1) * W + (h < TY ? TX + 1 : 0);
-  } else {
-    const int c = (h - 2 * TY) & (TX - 1), up = (h - 2 * TY) >> LX;
-    ih = min(x0 + c, nx) + sy * (up ? min(y0 + TY, ny) : y0 - 1);
-    hi = (up ? (TY + 1) * W : 0) + c + 1;
+  if (halo) {
+    int2 c;
+    if (h < 2 * TY) {
+      const bool right = h < TY;
+      const int r = right ? h : h - TY;
+      c.x = (right ? min(x0 + TX, nx) : x0 - 1) + sy * min(y0 + r, ny);
+      c.y = (r + 1) * W + (right ? TX + 1 : 0);
+    } else {
+      const bool above = h >= 2 * TY + TX;
+      const int q = h - 2 * TY - (above ? TX : 0);
+      c.x = min(x0 + q, nx) + sy * (above ? min(y0 + TY, ny) : y0 - 1);
+      c.y = (above ? (TY + 1) * W : 0) + q + 1;
+    }
+    sm.halo[h] = c;  // (read by this thread only)
   }
   // the extra faces: the first TX threads those above the tile, the next TY those right of it
   const bool up = tid < TX;
@@ -267,8 +284,9 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared<LX>& sm, const P
     const SoftVal X0 = stage(b, si, tc);
     X = stage(b ^ 1, si, tn);
     if (halo) {
-      stage(b, hi, __ldg(t0 + ih));
-      stage(b ^ 1, hi, __ldg(t0 + sz + ih));
+      const int2 c = sm.halo[h];
+      stage(b, c.y, __ldg(t0 + c.x));
+      stage(b ^ 1, c.y, __ldg(t0 + sz + c.x));
     }
     __syncthreads();
     bool ok;
@@ -278,21 +296,26 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared<LX>& sm, const P
     const SoftVal ay = staged(b, si - W);
     fy = softfp::soft_flux(s, ay, X0, ok);
     if (!ok) fy = hard(ay, X0);
-    sm.fx[b][ty * (TX + 1) + tx] = fx;
-    sm.fy[b][ty * TX + tx] = fy;
+    sm.fx[b][fi] = fx;
+    sm.fy[b][gi] = fy;
     extra(b);
     tn2 = __ldg(tin + (long)sz * min(z0 + 2, nz) + ic);
   }
+  const bool active = in_tile && x0 + tx < nx && y0 + ty < ny;
+  const bool edge = x0 + tx == 0 || x0 + tx == nx - 1 || y0 + ty == 0 || y0 + ty == ny - 1;
   auto store = [&](int z, double v) {
-    const int x = x0 + tx, y = y0 + ty;
-    if (x < nx && y < ny) store_images(tout, sy, (long)sz, x, y, z, nx, ny, nz, v);
+    if (!active) return;
+    if (edge || z == 0 || z == P.nz - 1)
+      store_images(tout, sy, (long)sz, it.x0 + tx, it.y0 + ty, z, P.nx, P.ny, P.nz, v);
+    else
+      tout[(long)sz * z + ic] = v;
   };
 #pragma unroll 1
   for (int z = z0;; ++z) {
     __syncthreads();
     const int buf = z & 1, nb = buf ^ 1;
-    const double a = __dsub_rn(sm.fx[buf][ty * (TX + 1) + tx + 1], fx);
-    const double b = __dsub_rn(sm.fy[buf][(ty + 1) * TX + tx], fy);
+    const double a = __dsub_rn(sm.fx[buf][fi + 1], fx);
+    const double b = __dsub_rn(sm.fy[buf][gi + TX], fy);
     const double c = __dsub_rn(fzhi, fzlo);
     if (z + 1 >= z1) {
       store(z, __dadd_rn(tc, __dmul_rn(hdt, __dadd_rn(__dadd_rn(a, b), c))));
@@ -308,7 +331,10 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared<LX>& sm, const P
     const double sum = __dadd_rn(ab, c);
     // plane z + 2 (exists: z + 1 < z1 <= nz)
     const SoftVal Xn = stage(buf, si, tn2);
-    if (halo) stage(buf, hi, __ldg(tin + (long)sz * (z + 2) + ih));
+    if (halo) {
+      const int2 c = sm.halo[h];
+      stage(buf, c.y, __ldg(tin + (long)sz * (z + 2) + c.x));
+    }
     const double prod = __dmul_rn(hdt, sum);
     const double gz = __dmul_rn(s, dz);
     const double v = __dadd_rn(tc, prod);
@@ -316,12 +342,12 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared<LX>& sm, const P
       gx = hard(xl, X);
       gy = hard(yl, X);
     }
-    sm.fx[nb][ty * (TX + 1) + tx] = gx;
-    sm.fy[nb][ty * TX + tx] = gy;
+    sm.fx[nb][fi] = gx;
+    sm.fy[nb][gi] = gy;
     extra(nb);
     tc = tn;
     tn = tn2;
-    tn2 = __ldg(tin + (long)sz * min(z + 3, nz) + ic);  // past nz: read again, not used
+    tn2 = __ldg(tin + (long)sz * min(z + 3, P.nz) + ic);  // past nz: read again, not used
     store(z, v);
     fx = gx;
     fy = gy;
@@ -335,17 +361,15 @@ __global__ void __launch_bounds__(PT_THREADS, 4) patches_soft_kernel(const Patch
                                                                      const WorkItem* __restrict__ items, int nitems,
                                                                      const double* __restrict__ src,
                                                                      double* __restrict__ dst) {
-  __shared__ PatchSoftAny sm;
+  __shared__ PatchSoftShared sm;
   step_begin();
   for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
-    const WorkItem it = items[w];
-    const PatchDev P = patches[it.patch];
-    if (P.log2tx == 4)
-      patch_soft_item<4>(sm.s4, P, it, src, dst);
-    else if (P.log2tx == 5)
-      patch_soft_item<5>(sm.s5, P, it, src, dst);
-    else
-      patch_soft_item<6>(sm.s6, P, it, src, dst);
+    if (threadIdx.x == 0) {
+      sm.it = items[w];
+      sm.P = patches[sm.it.patch];
+    }
+    __syncthreads();
+    patch_soft_item(sm, src, dst);
     __syncthreads();  // the staged planes and faces are reused by the next item
   }
   step_end();
@@ -778,6 +802,7 @@ std::vector<WorkItem> build_items(const PatchSet& ps, const std::vector<int>& wh
     const int nx = ps.shape[3 * p], ny = ps.shape[3 * p + 1], nz = ps.shape[3 * p + 2];
     // FP32: row strips (strip_shape); otherwise tiles, one row per thread row
     int TX = 1 << ps.log2tx[p], TY = PT_THREADS / TX;
+    if (ps.dtype == NEBO_F64 && !ps.wide_plane) tile_shape(nx, ny, ps.log2tx[p], TX, TY);
     if (ps.dtype == NEBO_F32) {
       if (ps.bulk32) {
         TX = nx;
@@ -793,6 +818,16 @@ std::vector<WorkItem> build_items(const PatchSet& ps, const std::vector<int>& wh
   // largest z-extent items first so the strided assignment ends with short items
   std::stable_sort(items.begin(), items.end(), [](const WorkItem& a, const WorkItem& b) { return (a.z1 - a.z0) > (b.z1 - b.z0); });
   return items;
+}
+
+// FP64 items' z extent: the longest of 48, 32 and 16 planes that leaves three waves of resident
+// blocks (an item stages two planes beyond its own; too few items leave the last wave ragged): 128
+// patches of 16..96 cells 5.53 ms per 10 steps at 48, 5.64 at 32, 5.78 at 16; 20 small ones 0.43 at 16,
+// 0.70 at 48.
+int f64_zchunk(const PatchSet& ps, const std::vector<int>& all) {
+  for (int zc : {48, 32})
+    if ((long)build_items(ps, all, zc).size() >= 3L * 4 * num_sms()) return zc;
+  return 16;
 }
 
 int upload_tables(PatchSet& ps, const std::vector<WorkItem>& items, cudaStream_t s) {
@@ -979,6 +1014,7 @@ extern "C" int nebo_patchset_create(nebo_patchset** out, int npatch, const int32
   }
   std::vector<int> all(npatch);
   for (int p = 0; p < npatch; ++p) all[p] = p;
+  if (dtype == NEBO_F64) ps->zchunk = f64_zchunk(*ps, all);
   int rc = upload_tables(*ps, build_items(*ps, all, ps->zchunk), 0);
   if (rc) {
     delete ps;
@@ -1146,6 +1182,7 @@ extern "C" int nebo_patchset_autotune(nebo_patchset* ps, nebo_stream_t stream, i
   if (rc) return rc;
   std::vector<int> all(ps->npatch);
   for (int p = 0; p < ps->npatch; ++p) all[p] = p;
+  if (ps->dtype == NEBO_F64) ps->zchunk = f64_zchunk(*ps, all);
   rc = upload_tables(*ps, build_items(*ps, all, ps->zchunk), s);
   if (rc) return rc;
   if (chosen_log2tx)
