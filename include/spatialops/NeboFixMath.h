@@ -16,8 +16,9 @@
 //     the nearest works); r1 = x - k*L1 exactly in FP64 (L1 = ln2/256 to 35 bits, so k*L1 is exact
 //     for |k| < 2^18); r = r1 - k*L2 in fixed point (L2 = ln2/256 - L1 to 2^-104).  The inner
 //     factors 1/24 + r/120 (FP32) and 1/6 + r*(...), 1/2 + r*(...) (32x32-bit products) need few
-//     bits; r^2, r^2*(...) and 2^(j/256)*(1 + p) are 64-bit products; the result is rounded to a
-//     double from the 62-fraction-bit fixed point.
+//     bits; r^2, r^2*(...) and 2^(j/256)*(1 + p) are 64-bit products of which only the high half
+//     is formed (r is held at 2^72: |r| < 2^-9.5 leaves those halves more bits than the final
+//     rounding needs); the result is rounded to a double from the 62-fraction-bit fixed point.
 // sin(x), |x| < 2^20  x = k pi/256 + r,  |r| <= pi/512 (+1 % from the FP32 rounding of k):
 //     sin(x) = S_k (1 + (cos r - 1)) + C_k sin r,  S_k, C_k = sin, cos(k pi/256) from a 128-entry
 //     quarter table and the quadrant of k;  sin r = r (1 - u/6 + u^2/120),
@@ -29,7 +30,16 @@
 //     and sin r = r * (1 - u/6 + u^2/120) is a product of r's significand.
 // Everything else -- |x| beyond those ranges, NaN, infinities -- goes to CUDA's exp and sin.
 //
-// Fixed point: signed or unsigned 64-bit integers with 62 fraction bits ("at 2^62").  Error: exp
+// Products of signed quantities are formed on magnitudes: one 64x64 high half is five 32-bit
+// multiply-adds, while a signed one, or one shifted across both halves, is eight to ten, and
+// products are most of the instructions.  The deep chain's kernel (one exp, one sin and a
+// four-point stencil a cell, bound by the integer pipes: ALU 74 % busy) takes 271 us at 256^3;
+// with signed full products at 2^62 throughout it took 346 us.  The error fell with it, because
+// r keeps eight to ten more bits (exp 0.513 -> 0.506 ulp, sin away from multiples of pi
+// 0.84 -> 0.63, over two million arguments each).
+//
+// Fixed point: signed or unsigned 64-bit integers with 62 fraction bits ("at 2^62") unless a
+// value's own scale is named beside it.  Error: exp
 // within 0.52 ulp, sin within about 1.1 ulp (the FP64 rounding of r before the final rounding in
 // the multiple-of-pi branch; fixed-point roundings where |sin x| is near sin(pi/512), whose ulp is
 // 4 units of 2^-62); the tests compare both with long double on the host and with CUDA's
@@ -116,46 +126,15 @@ __host__ __device__ __forceinline__ int fbits(float x) {
 }
 __host__ __device__ __forceinline__ uint64_t uabs(int64_t a) { return a < 0 ? 0 - (uint64_t)a : (uint64_t)a; }
 
-// a * b / 2^62 for a, b >= 0: high word only (truncation below 4 units of 2^-62), and rounded to
-// nearest (the full 128-bit product plus one half, a < 2^64, a * b < 2^126).  ssq: a^2 / 2^62
-// truncated like umulq, from the signed high word (a^2 = |a|^2, so the same bits as umulq(|a|, |a|)).
-__host__ __device__ __forceinline__ uint64_t umulq(uint64_t a, uint64_t b) { return umulhi(a, b) << 2; }
-__host__ __device__ __forceinline__ uint64_t ssq(int64_t a) {
-#ifdef __CUDA_ARCH__
-  return (uint64_t)__mul64hi(a, a) << 2;
-#else
-  return (uint64_t)(((__int128)a * (__int128)a) >> 64) << 2;
-#endif
-}
-__host__ __device__ __forceinline__ uint64_t umulx(uint64_t a, uint64_t b) {
-  const uint64_t lo = a * b, lo2 = lo + (1ULL << 61);
-  return ((umulhi(a, b) + (lo2 < lo)) << 2) | (lo2 >> 62);
-}
-// signed a * b / 2^62 rounded to nearest (halves up), from the signed 128-bit product
-// (|a * b| < 2^125)
-__host__ __device__ __forceinline__ int64_t smulx(int64_t a, int64_t b) {
-#ifdef __CUDA_ARCH__
-  const uint64_t lo = (uint64_t)a * (uint64_t)b;
-  const int64_t hi = __mul64hi(a, b);
-#else
-  const __int128 pr = (__int128)a * (__int128)b;
-  const uint64_t lo = (uint64_t)pr;
-  const int64_t hi = (int64_t)(pr >> 64);
-#endif
-  const uint64_t lo2 = lo + (1ULL << 61);
-  const uint64_t hi2 = (uint64_t)hi + (lo2 < lo);
-  return (int64_t)((hi2 << 2) | (lo2 >> 62));
-}
-
-// A finite double with |v| < 2 at 2^62 (truncated toward zero; 0 for subnormals).
-__host__ __device__ __forceinline__ int64_t to_fix(double v) {
+// A double at 2^S modulo 2^64, truncated toward zero (|v| 2^S < 2^64; 0 for subnormals).
+template <int S>
+__host__ __device__ __forceinline__ int64_t to_fix_small(double v) {
   const uint64_t b = bits(v);
   const int e = (int)((b >> 52) & 0x7ff);
-  const uint64_t m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL;
-  const int sh = e - 1013;  // v = m * 2^(e - 1075)
-  uint64_t f = sh >= 0 ? m << sh : (sh > -64 ? m >> -sh : 0);
-  if (e == 0) f = 0;
-  return (b >> 63) ? -(int64_t)f : (int64_t)f;
+  const uint64_t m = ((b & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;  // v = m 2^(e - 1086)
+  const int sh = 1086 - S - e;
+  const uint64_t f = m >> (sh < 63 ? sh : 63);  // (a zero's m has its top bit alone above the shift)
+  return (int64_t)b < 0 ? -(int64_t)f : (int64_t)f;
 }
 
 // k * C / 2^S for a signed 32-bit k and a 62-bit signed constant C, 32 <= S < 64, rounded
@@ -265,33 +244,27 @@ __host__ __device__ __forceinline__ double exp_fix(double x, const T& tb) {
   double kd;
   const int k = k_f32(x, 369.32992553710938f, &kd);  // 256/ln2
   const double r1 = fma(-kd, L1, x);                  // exact
-  const int64_t r = to_fix(r1) - mul_k<42>(k, L2_FIX104);
+  // r at 2^72 (|r| < 2^-9.5): its high word is r at 2^40, and the high halves of its products need no
+  // low halves to be rounded well below 2^-62
+  const int64_t r = to_fix_small<72>(r1) - mul_k<32>(k, L2_FIX104);
   // g2 = 1/24 + r/120 in FP32, in [2^-5, 2^-4): its significand at 2^35 is exact
   const float g2 = fmaf(f32_trunc(r1), 1.0f / 120.0f, 1.0f / 24.0f);
   const int32_t g2f = (int32_t)(((uint32_t)fbits(g2) & 0x7fffffu) | 0x800000u) << 7;
-  const int32_t r40 = (int32_t)(r >> 22);  // r at 2^40
+  const int32_t r40 = (int32_t)(r >> 32);
   const int64_t g = SIXTH + (((int64_t)r40 * g2f) >> 13);               // 1/6 + r g2
   const int64_t h = HALF + (((int64_t)r40 * (int32_t)(g >> 30)) >> 10);  // 1/2 + r g
-  const uint64_t u = ssq(r);                                            // r^2
-  const int64_t p = r + (int64_t)umulq(u, (uint64_t)h);
+  const uint64_t a = uabs(r);
+  const uint64_t u = umulhi(a, a);                                       // r^2 at 2^80
+  const int64_t p = r + (int64_t)(umulhi(u, (uint64_t)h) >> 6);          // at 2^72
   const int64_t tj = tb.e(k & 255);
-  const uint64_t y = (uint64_t)(tj + smulx(tj, p));
-  return from_bits(fix_to_bits(y, k >> 8));
+  const int64_t tp = (int64_t)umulhi((uint64_t)tj, (uint64_t)p) - (tj & (p >> 63));  // tj p at 2^70
+  const uint64_t y = (uint64_t)(tj + ((tp + 128) >> 8));  // in [2^61, 2^63)
+  const uint64_t yn = y << (2 - (int)(y >> 62));          // top bit at 63
+  const uint64_t m = (yn >> 11) + ((yn >> 10) & 1);
+  return from_bits(((uint64_t)((k >> 8) + 1021 + (int)(y >> 62)) << 52) + m);
 }
 
 // ------------------------------------------------------------------ sin
-// -u/6 + u^2/120 and cos r - 1 = -u/2 + u^2/24 - u^3/720 at 2^62, from u = r^2 at 2^62 (u < 2^-14)
-__host__ __device__ __forceinline__ void sin_cos_poly(uint64_t u, int64_t* sfac_m1, int64_t* cm1) {
-  const uint32_t u46 = (uint32_t)(u >> 16);                          // u at 2^46
-  const uint32_t uu60 = (uint32_t)(((uint64_t)u46 * u46) >> 32);      // u^2 at 2^60
-  const int64_t u2_120 = (int64_t)(((uint64_t)uu60 * C120) >> 30);    // u^2/120 at 2^62
-  const int64_t u2_24 = (int64_t)(((uint64_t)uu60 * C24) >> 30);      // u^2/24
-  const uint64_t u3 = ((uint64_t)uu60 * u46) >> 44;                   // u^3 at 2^62
-  const int64_t u3_720 = (int64_t)((u3 * C720) >> 32);               // u^3/720
-  *sfac_m1 = -(int64_t)umulhi(u, SIXTH64) + u2_120;
-  *cm1 = -(int64_t)(u >> 1) + u2_24 - u3_720;
-}
-
 template <class T>
 __host__ __device__ __forceinline__ double sin_fix(double x, const T& tb) {
   const uint64_t xb = bits(x);
@@ -314,6 +287,15 @@ __host__ __device__ __forceinline__ double sin_fix(double x, const T& tb) {
   }
   const double r1 = fma(-kd, A1, x);  // exact
   const int q = (k >> 7) & 3;
+  const int64_t r = to_fix_small<62>(r1) - mul_k<32>(k, A23_FIX94);
+  // |r| at 2^70 (below 2^-7.3), u = r^2 at 2^76; 1 - sin|r|/|r| and 1 - cos r at 2^76, so that the
+  // high halves of the products need no low halves to be rounded well below 2^-62
+  const uint64_t a = uabs(r) << 8;
+  const uint64_t u = umulhi(a, a);
+  const uint32_t u46 = (uint32_t)(u >> 30);
+  const uint32_t uu60 = (uint32_t)(((uint64_t)u46 * u46) >> 32);          // u^2 at 2^60
+  const uint32_t u3 = (uint32_t)(((uint64_t)uu60 * u46) >> 31);           // u^3 at 2^75
+  const uint64_t sm = umulhi(u, SIXTH64) - (((uint64_t)uu60 * C120) >> 16);  // u/6 - u^2/120
   if ((k & 255) == 0) {
     // +-sin r, r possibly tiny: r in FP64 with pi/256 in four parts, then r * (1 - u/6 + u^2/120)
     double rd = r1;  // k = 0: r = x exactly (keeps the sign of -0)
@@ -325,10 +307,7 @@ __host__ __device__ __forceinline__ double sin_fix(double x, const T& tb) {
     const uint64_t rb = bits(rd) ^ ((uint64_t)(q >> 1) << 63);  // sin(r + pi) = -sin r
     const int er = (int)((rb >> 52) & 0x7ff);
     if (er < 1023 - 26) return from_bits(rb);                   // |r| < 2^-26: sin r = r
-    const uint64_t ra = uabs(to_fix(rd));
-    int64_t sm1, cm1;
-    sin_cos_poly(umulq(ra, ra), &sm1, &cm1);
-    const uint64_t s = (uint64_t)(ONE + sm1);                   // 1 - u/6 + u^2/120 <= 2^62
+    const uint64_t s = (uint64_t)ONE - (sm >> 14);              // 1 - u/6 + u^2/120 <= 2^62
     const uint64_t mr = ((rb & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;  // top bit 63
     const uint64_t pr = umulhi(mr, s << 1);                    // top bit at 61..63
     const int lz = clz64(pr);
@@ -337,18 +316,19 @@ __host__ __device__ __forceinline__ double sin_fix(double x, const T& tb) {
     // sin r = (pn / 2^63) * 2^(er - 1022 - lz); m's implicit bit adds one to the exponent field
     return from_bits((rb & 0x8000000000000000ULL) | (((uint64_t)(er - lz) << 52) + m));
   }
-  const int64_t r = to_fix(r1) - mul_k<32>(k, A23_FIX94);
-  int64_t sm1, cm1;
-  sin_cos_poly(ssq(r), &sm1, &cm1);
-  const int64_t sr = r + smulx(r, sm1);  // sin r
+  const uint64_t cm = (u >> 1) - (((uint64_t)uu60 * C24) >> 16) + (((uint64_t)u3 * C720) >> 31);  // 1 - cos r
+  const uint64_t sr = a - (umulhi(a, sm) >> 12);  // sin|r| at 2^70
+  // With S, C the sine and cosine of j pi/256 (swapped in odd quadrants), the result is
+  // (-1)^(q/2) (S cos r +- C sin|r|), the inner sign that of r, turned in odd quadrants; S exceeds
+  // C sin|r| here (j > 0 or S = 1), so the sum is positive.
   const int j = k & 127;
   const int64_t sj = tb.s(j), cj = tb.c(j);
-  int64_t sk = (q & 1) ? cj : sj, ck = (q & 1) ? sj : cj;
-  if (q & 2) sk = -sk;
-  if ((q ^ (q >> 1)) & 1) ck = -ck;
-  const int64_t v = sk + smulx(sk, cm1) + smulx(ck, sr);
-  const uint64_t sign = (uint64_t)v & 0x8000000000000000ULL;
-  return from_bits(sign | fix_to_bits(uabs(v), 0));
+  const int64_t S = (q & 1) ? cj : sj, C = (q & 1) ? sj : cj;
+  const int64_t t = (int64_t)umulhi((uint64_t)C, sr);                 // at 2^68
+  const int64_t w = (int64_t)(umulhi((uint64_t)S, cm) >> 6);          // at 2^68
+  const bool minus = (r < 0) != ((q & 1) != 0);
+  const int64_t v = S + (((minus ? -t : t) - w + 32) >> 6);
+  return from_bits(((uint64_t)(q >> 1) << 63) | fix_to_bits((uint64_t)v, 0));
 }
 
 
