@@ -173,12 +173,18 @@ constexpr int FTY = 16;  // filter tile y (each thread of the 32 x 8 block owns 
 // four reductions of the values written (one Acc4 partial per block).
 //
 // Planes of `out` (the 32 x 16 tile plus a one-cell halo) stream through a ring of FNS
-// shared-memory stages with cp.async.  Ring schedule: plane p (-1..nz) lives in stage
-// (p+1) % FNS; the prologue issues planes z0-1 .. z0+FNS-3; iteration p waits until plane p has
-// landed (at most FNS-2 groups pending), syncs, issues plane p+FNS-1 into the stage of plane p-1
-// (consumed in iteration p-1, before the sync), then sums plane p: x-sums of 3 into `rows`
-// (two neighbouring sums share their middle pair), a sync, y-sums of 3 for the thread's two
-// cells; the 2-D sums of planes p-2, p-1, p give the outputs of plane p-1.
+// shared-memory stages with cp.async.  Plane p (-1..nz) lives in stage (p+1) % FNS.  A thread
+// converts the values it copied itself, so a landed plane needs no barrier: iteration p issues
+// plane p+FNS-1 into the stage of plane p-1, waits until its own part of plane p+1 has landed,
+// folds that plane's largest exponent and converts plane p into `fplane` (its largest exponent
+// is known from the iteration before); a barrier; x-sums of 3 into `rows` (two neighbouring sums
+// share their middle pair); a barrier; y-sums of 3 for the thread's two cells.  The 2-D sums of
+// three planes give the outputs of the middle one, formed in the next iteration beside its
+// integer conversions (the FP64 pipe is the busiest: 65 % at 256^3, ALU 47 %).  `fplane` and the exponents of p are read
+// before the second barrier and written after it; `rows` is read after it and written after the
+// next iteration's first.  256^3 with the reductions: 239 us (262 us with four barriers a plane,
+// 64-bit shifts in the conversions and the outputs formed at once; 247 us at five blocks an SM,
+// whose 48 registers spill).
 //
 // The 9-point (x, y) sums of a plane run on the integer pipe, exactly, in 128-bit fixed point
 // (fp64_int.cuh).  A plane whose largest biased exponent is E converts each value to an integer
@@ -238,48 +244,66 @@ __global__ void __launch_bounds__(FX* FY, 4) box_filter_kernel(const double* __r
         cp_async8(st + soff[j], sp + goff[j]);
       }
     };
+    // largest biased exponent of plane p, from the values this thread copied, into its slot
+    auto scan = [&](int p) {
+      const double* pl = ring + ((p + 1) % FNS) * PLANE;
+      unsigned e = 0;
+#pragma unroll
+      for (int j = 0; j < NCOPY; ++j) {
+        const int t = tid + j * FX * FY;
+        if (t < PLANE) e = max(e, ((unsigned)__double2hiint(pl[t]) >> 20) & 0x7ffu);
+      }
+      e = __reduce_max_sync(0xffffffffu, e);
+      if (lane == 0) atomicMax(&plane_exp[p & 1], e);
+    };
     if (tid < 2) plane_exp[tid] = 0u;
 #pragma unroll 1
     for (int i = 0; i < FNS - 1; ++i) {
       issue(z0 - 1 + i);
       cp_async_commit();
     }
+    cp_async_wait<FNS - 2>();
+    __syncthreads();
+    scan(z0 - 1);
+    __syncthreads();
     const bool act0 = x < nx && ya < ny, act1 = x < nx && ya + 1 < ny;
-    // 9-point (x, y) sums of planes p-2 (p*) and p-1 (c*) for both cells
-    double p0 = 0.0, c0 = 0.0, p1 = 0.0, c1 = 0.0;
-    double* out = dst + (long)x + (long)sy * ya + sz * (z0 - 1);
+    // 9-point (x, y) sums of planes p-3 (p*), p-2 (c*) and p-1 (s*) for both cells
+    double p0 = 0.0, c0 = 0.0, s0 = 0.0, p1 = 0.0, c1 = 0.0, s1 = 0.0;
+    double* out = dst + (long)x + (long)sy * ya + sz * z0;
+    auto emit = [&]() {  // the outputs of the plane that c* belongs to
+      constexpr double C27 = 1.0 / 27.0;
+      const double v0 = __dmul_rn(__dadd_rn(__dadd_rn(p0, c0), s0), C27);
+      const double v1 = __dmul_rn(__dadd_rn(__dadd_rn(p1, c1), s1), C27);
+      if (act0) {
+        *out = v0;
+        if (RED) acc4_add(acc, v0);
+      }
+      if (act1) {
+        out[sy] = v1;
+        if (RED) acc4_add(acc, v1);
+      }
+      out += sz;
+    };
 #pragma unroll 1
-    for (int p = z0 - 1; p <= z1; ++p, out += sz) {
-      cp_async_wait<FNS - 2>();
-      __syncthreads();
+    for (int p = z0 - 1; p <= z1; ++p) {
       issue(p + FNS - 1);
       cp_async_commit();
+      cp_async_wait<FNS - 2>();  // this thread's part of plane p+1 has landed
       const double* pl = ring + ((p + 1) % FNS) * PLANE;
-      // the plane's largest biased exponent; this thread's values stay in registers
-      constexpr int PER = (PLANE + FX * FY - 1) / (FX * FY);
-      double val[PER];
-      unsigned e = 0;
-#pragma unroll
-      for (int j = 0; j < PER; ++j) {
-        const int t = tid + j * FX * FY;
-        val[j] = t < PLANE ? pl[t] : 0.0;
-        e = max(e, ((unsigned)__double2hiint(val[j]) >> 20) & 0x7ffu);
-      }
-      e = __reduce_max_sync(0xffffffffu, e);
-      if (lane == 0) atomicMax(&plane_exp[p & 1], e);
-      __syncthreads();
       const int E = (int)plane_exp[p & 1];
-      if (tid == 0) plane_exp[(p + 1) & 1] = 0u;  // the slot of plane p+1 (last read in iteration p-1)
       const bool special = E == 0x7ff || E < 130 || E > 2040;
       const int u = E - 1144;
+      if (p < z1) scan(p + 1);
+      if (p >= z0 + 2) emit();
       if (!special) {
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
+        for (int j = 0; j < NCOPY; ++j) {
           const int t = tid + j * FX * FY;
-          if (t < PLANE) fplane[t] = fixmath::to_units(val[j], E);
+          if (t < PLANE) fplane[t] = fixmath::to_units(pl[t], E);
         }
-        __syncthreads();
       }
+      __syncthreads();
+      if (tid == 0) plane_exp[p & 1] = 0u;  // every thread has read it: the slot of plane p+2
       for (int t = tid; t < XTASKS; t += FX * FY) {
         const int r = t / (FX / 2), c = 2 * (t % (FX / 2));
         if (!special) {
@@ -296,7 +320,10 @@ __global__ void __launch_bounds__(FX* FY, 4) box_filter_kernel(const double* __r
       }
       __syncthreads();
       const fixmath::fix128* col = rows + 2 * ty * FX + tx;
-      double s0, s1;
+      p0 = c0;
+      c0 = s0;
+      p1 = c1;
+      c1 = s1;
       if (!special) {
         const fixmath::fix128 mid = col[FX] + col[2 * FX];
         s0 = fixmath::units_to_double0(col[0] + mid, u);
@@ -307,24 +334,8 @@ __global__ void __launch_bounds__(FX* FY, 4) box_filter_kernel(const double* __r
         s0 = __dadd_rn(d(col[0]), mid);
         s1 = __dadd_rn(mid, d(col[3 * FX]));
       }
-      if (p >= z0 + 1) {
-        constexpr double C27 = 1.0 / 27.0;
-        if (act0) {
-          const double v = __dmul_rn(__dadd_rn(__dadd_rn(p0, c0), s0), C27);
-          out[-sz] = v;  // plane p-1
-          if (RED) acc4_add(acc, v);
-        }
-        if (act1) {
-          const double v = __dmul_rn(__dadd_rn(__dadd_rn(p1, c1), s1), C27);
-          out[sy - sz] = v;
-          if (RED) acc4_add(acc, v);
-        }
-      }
-      p0 = c0;
-      c0 = s0;
-      p1 = c1;
-      c1 = s1;
     }
+    emit();
     cp_async_wait<0>();
     __syncthreads();  // the ring and plane_exp are free for the next run
   }

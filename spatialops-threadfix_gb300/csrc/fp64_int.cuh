@@ -28,58 +28,69 @@ __host__ __device__ __forceinline__ fix128 make128(long long hi, unsigned long l
   return (fix128)(((unsigned __int128)(unsigned long long)hi << 64) | lo);
 }
 
+// The top word of (hi : lo) << s, 0 <= s < 32.
+__host__ __device__ __forceinline__ uint32_t fsl32(uint32_t lo, uint32_t hi, int s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, s);
+#else
+  return (uint32_t)(((((uint64_t)hi << 32) | lo) << s) >> 32);
+#endif
+}
+
 // x (biased exponent <= E, not inf/NaN) in units of 2^(E-1144), rounded to nearest (halves up):
-// the 53-bit significand m lands at bit sh = e - E + 69 <= 69 of a 128-bit integer.
+// the 53-bit significand m lands at bit sh = e - E + 69 <= 69 of a 128-bit integer.  In 32-bit
+// words: one shift by sh mod 32 across the significand's two words and a choice of the word they
+// start at (64-bit shifts by a variable count are several instructions each).
 __host__ __device__ __forceinline__ fix128 to_units(double x, int E) {
   const long long b = (long long)bits(x);
   const int e = (int)((b >> 52) & 0x7ff);
-  const unsigned long long m = ((unsigned long long)b & 0xFFFFFFFFFFFFFull) | (e ? (1ull << 52) : 0ull);
-  const int sh = (e ? e : 1) - E + 69;
-  unsigned long long hi, lo;
-  if (sh >= 64) {
-    hi = m << (sh - 64);
-    lo = 0;
-  } else if (sh > 0) {
-    hi = m >> (64 - sh);
-    lo = m << sh;
-  } else {
-    hi = 0;
-    lo = sh == 0 ? m : (-sh > 62 ? 0ull : (m + (1ull << (-sh - 1))) >> -sh);
+  unsigned long long m = ((unsigned long long)b & 0xFFFFFFFFFFFFFull) | (e ? (1ull << 52) : 0ull);
+  int sh = (e ? e : 1) - E + 69;
+  if (sh < 0) {
+    m = sh < -62 ? 0ull : (m + (1ull << (-sh - 1))) >> -sh;
+    sh = 0;
   }
-  const fix128 f = make128((long long)hi, lo);
-  return b < 0 ? -f : f;
+  const unsigned long long ms = b < 0 ? 0ull - m : m;
+  const uint32_t m0 = (uint32_t)ms, m1 = (uint32_t)(ms >> 32), sg = (uint32_t)((int32_t)m1 >> 31);
+  const int s = sh & 31;
+  const bool q0 = sh < 32, q1 = sh < 64;
+  const uint32_t t0 = m0 << s, t1 = fsl32(m0, m1, s), t2 = fsl32(m1, sg, s);
+  const uint32_t w0 = q0 ? t0 : 0u, w1 = q0 ? t1 : (q1 ? t0 : 0u);
+  const uint32_t w2 = q0 ? t2 : (q1 ? t1 : t0), w3 = q0 ? sg : (q1 ? t2 : t1);
+  return make128((long long)(((uint64_t)w3 << 32) | w2), ((uint64_t)w1 << 32) | w0);
 }
 
-// RN(t 2^u) for t != 0, assuming the result is normal.
+// RN(t 2^u) for t != 0, assuming the result is normal.  In 32-bit words: the leading bit's word
+// is moved to the top (usually it is there), one funnel shift a word normalises, and the rounding
+// increment carries into the exponent field by itself.
 __host__ __device__ __forceinline__ double units_to_double(fix128 t, int u) {
   const bool neg = t < 0;
   const unsigned __int128 a = neg ? (unsigned __int128)(-t) : (unsigned __int128)t;
-  const unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
-  unsigned long long top, rest;
-  int msb;  // position of the leading bit
-  if (hi) {
-    const int lz = clz64(hi);
-    top = lz ? (hi << lz) | (lo >> (64 - lz)) : hi;
-    rest = lo << lz;  // bits below `top` (only whether any is set matters)
-    msb = 127 - lz;
-  } else {
-    const int lz = clz64(lo);
-    top = lo << lz;
-    rest = 0;
-    msb = 63 - lz;
+  uint32_t w3 = (uint32_t)(a >> 96), w2 = (uint32_t)(a >> 64), w1 = (uint32_t)(a >> 32), w0 = (uint32_t)a;
+  int ex = 127 + u + 1023;  // biased exponent of bit 127
+  if (w3 == 0u) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (w3 == 0u) {
+        w3 = w2;
+        w2 = w1;
+        w1 = w0;
+        w0 = 0u;
+        ex -= 32;
+      }
   }
-  unsigned long long mant = top >> 11;  // 53 bits
-  const unsigned long long rb = top & 0x7ffull;
-  const bool up = rb > 0x400ull || (rb == 0x400ull && (rest != 0 || (mant & 1ull)));
-  int ex = msb + u + 1023;
-  mant += up ? 1ull : 0ull;
-  if (mant >> 53) {
-    mant >>= 1;
-    ++ex;
-  }
-  const unsigned long long out = ((unsigned long long)neg << 63) | ((unsigned long long)ex << 52) |
-                                 (mant & 0xFFFFFFFFFFFFFull);
-  return from_bits(out);
+#ifdef __CUDA_ARCH__
+  const int lz = __clz((int)w3);
+#else
+  const int lz = clz64(w3) - 32;
+#endif
+  const uint32_t h = fsl32(w2, w3, lz), l = fsl32(w1, w2, lz);
+  const bool sticky = (fsl32(w0, w1, lz) | (w0 << lz)) != 0u;
+  const uint32_t mh = h >> 11, ml = fsl32(l, h, 21);  // 53 bits, the leading one included
+  const uint32_t low = ((l & 0x7ffu) << 1) | (sticky ? 1u : 0u);
+  const uint32_t up = low + (ml & 1u) > 0x800u ? 1u : 0u;
+  const uint32_t top = (neg ? 0x80000000u : 0u) + ((uint32_t)(ex - lz - 1) << 20) + mh;
+  return from_bits((((uint64_t)top << 32) | ml) + up);
 }
 
 // RN(t 2^u), +0 for t == 0, assuming a nonzero result is normal.
