@@ -557,19 +557,24 @@ __global__ void __launch_bounds__(PT_THREADS, 2) patches_f32_strip_kernel(const 
 // FP32 mode on bulk-copied slabs (every patch with nx <= PB_CELLS).  The FP32 working state
 // holds each patch's interior only, rows padded to a multiple of 4 floats (16 bytes) and each
 // patch 256-byte aligned, so every row starts on a 16-byte boundary.  An item is a strip of R
-// full rows of one patch over a z range (R nx <= 1024, the rows split evenly between the strips).
+// full rows of one patch over a z range (the rows split evenly between the strips).
 // Per plane three cp.async.bulk copies fill a stage of the ring: the row below the strip, its R
 // rows (one contiguous run) and the row above, the two halo rows and the halo planes taken from
 // their periodic sources (rows ny-1 / 0, planes nz-1 / 0); the x halo is the row's own other end.
-// One thread arms the stage's mbarrier and issues the copies; the 256 threads own the strip's
-// cells linearly (4 each) and compute what patches_f32_strip_kernel computes, with the same
-// operations.  No ghost cells exist in this layout: nebo_patchset_sync writes whole FP64 windows.
-constexpr int PB_CELLS = 1024;                 // cells per strip plane
-constexpr int PB_CPT = PB_CELLS / PT_THREADS;  // cells per thread
-constexpr int PB_NS = 5;                       // stages
+// One thread arms the stage's mbarrier and issues the copies; each of the 256 threads owns four
+// consecutive cells of a row (R pitch <= 1024): rows start on 16-byte boundaries, so the rows above,
+// below and of the next plane are one 16-byte load each and the four results one store, and only
+// the two cells beside the quad are single loads.  A thread with four cells 256 apart loaded each
+// neighbour of each cell by itself, 54 instructions a cell, and was bound by issue (81 %); 512
+// patches of 16..96 cells an edge (742 MB a step) took 170 us a step that way and take 122 us so
+// (6.1 TB/s; bound by memory; 131 us with three stages, 124 with five, 138 with seven, 134 at eight
+// blocks an SM, whose 32 registers spill).  The operations of a cell are those of patches_f32_strip_kernel in the same order.
+// No ghost cells exist in this layout: nebo_patchset_sync writes whole FP64 windows.
+constexpr int PB_CELLS = 4 * PT_THREADS;  // floats per strip plane, the rows' padding included
+constexpr int PB_NS = 4;                  // stages
 
 __host__ __device__ __forceinline__ int strip_rows_bulk(int nx, int ny) {
-  const int rmax = PB_CELLS / nx > 0 ? PB_CELLS / nx : 1;
+  const int rmax = PB_CELLS / ((nx + 3) / 4 * 4);
   const int nstrips = (ny + rmax - 1) / rmax;
   return (ny + nstrips - 1) / nstrips;
 }
@@ -606,12 +611,11 @@ __global__ void __launch_bounds__(PT_THREADS) patches_f32_bulk_kernel(const Patc
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // plane q of the item is z0 - 1 + q (periodic), in stage q % PB_NS, phase (q / PB_NS) & 1
-    auto issue = [&](int q) {
+    // plane q of the item is z0 - 1 + q (periodic), in stage st = q % PB_NS, phase (q / PB_NS) & 1
+    auto issue = [&](int q, int st) {
       const int p = z0 - 1 + q;
       if (p > z1) return;  // the last plane read is z1 (the +z neighbour of the item's last plane)
       const int pw = p < 0 ? p + nz : (p >= nz ? p - nz : p);
-      const int st = q % PB_NS;
       const uint32_t bar = bar0 + 8 * st;
       const uint32_t so = ring0 + (uint32_t)(st * stage_floats) * 4u;
       const float* pl = base + (long)pw * sz;
@@ -621,48 +625,53 @@ __global__ void __launch_bounds__(PT_THREADS) patches_f32_bulk_kernel(const Patc
       bulk_g2s(so + (uint32_t)(R + 1) * rowb, pl + (long)yhi * pitch, rowb, bar);
     };
     if (tid == 0)
-      for (int q = 0; q < PB_NS; ++q) issue(q);
-    // this thread's cells: strip cell tid + 256 j -> stage indices (centre, x-1, x+1, wrapped
-    // within the row) and the output offset in a plane; bit j of `live`: the cell exists
-    int si[PB_CPT], sl[PB_CPT], sr[PB_CPT], go[PB_CPT];
-    unsigned live = 0;
-#pragma unroll
-    for (int j = 0; j < PB_CPT; ++j) {
-      const int c = tid + j * PT_THREADS;
-      const bool in = c < R * nx;
-      const int r = in ? c / nx : 0, col = in ? c - r * nx : 0;
-      if (in) live |= 1u << j;
-      si[j] = (r + 1) * pitch + col;
-      sl[j] = (r + 1) * pitch + (col == 0 ? nx - 1 : col - 1);
-      sr[j] = (r + 1) * pitch + (col == nx - 1 ? 0 : col + 1);
-      go[j] = (it.y0 + r) * pitch + col;
-    }
+      for (int q = 0; q < PB_NS; ++q) issue(q, q);
+    // this thread's four cells of a row (fewer at the row's end: the row's last quad may hold
+    // padding, which is computed and stored but never read as a neighbour) in a stage; the cells
+    // left and right of them, wrapped within the row; cell `last` is the row's last one
+    const int quads = pitch >> 2;
+    const bool act = tid < R * quads;
+    const int r = act ? tid / quads : 0, col = act ? 4 * (tid - r * quads) : 0;
+    const int row = (r + 1) * pitch, si = row + col;
+    const int sl = row + (col == 0 ? nx : col) - 1, sr = col + 4 >= nx ? row : si + 4;
+    const int last = nx - 1 - col;
+    const float* mine = ring + si;
     ok &= mbar_wait(bar0, 0) & mbar_wait(bar0 + 8, 0);
-    float t[PB_CPT], tb[PB_CPT];  // the cell and the one below it
-#pragma unroll
-    for (int j = 0; j < PB_CPT; ++j) {
-      t[j] = ring[stage_floats + si[j]];
-      tb[j] = ring[si[j]];
-    }
+    float4 tb = *reinterpret_cast<const float4*>(mine);                // the cells below
+    float4 t = *reinterpret_cast<const float4*>(mine + stage_floats);  // the cells
+    float* op = obase + (long)z0 * sz + (it.y0 + r) * pitch + col;
+    int cs = 1, cn = 2, ce = 0;  // stages of the centre plane q, of q + 1 and of q - 1
+    uint32_t phase = 0;          // of stage cn
     for (int z = z0; z < z1; ++z) {
-      const int q = z - z0 + 1;  // centre plane
-      __syncthreads();           // plane q-1's stage is no longer read
+      __syncthreads();  // plane q-1's stage is no longer read
       if (tid == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        issue(q - 1 + PB_NS);
+        issue(z - z0 + PB_NS, ce);
       }
-      ok &= mbar_wait(bar0 + 8 * ((q + 1) % PB_NS), ((q + 1) / PB_NS) & 1);
-      const float* T0 = ring + (q % PB_NS) * stage_floats;
-      const float* Tn = ring + ((q + 1) % PB_NS) * stage_floats;
-      float* op = obase + (long)z * sz;
-#pragma unroll
-      for (int j = 0; j < PB_CPT; ++j) {
-        const int c = si[j];
-        const float tc = t[j], tn = Tn[c];
-        const float nb = ((T0[sl[j]] + T0[sr[j]]) + (T0[c - pitch] + T0[c + pitch])) + (tb[j] + tn);
-        if ((live >> j) & 1u) op[go[j]] = fmaf(k, fmaf(-6.0f, tc, nb), tc);
-        tb[j] = tc;
-        t[j] = tn;
+      ok &= mbar_wait(bar0 + 8 * cn, phase);
+      const float* T0 = ring + cs * stage_floats;
+      const float4 tn = *reinterpret_cast<const float4*>(mine + cn * stage_floats);
+      const float4 td = *reinterpret_cast<const float4*>(T0 + si - pitch);
+      const float4 tu = *reinterpret_cast<const float4*>(T0 + si + pitch);
+      const float tl = T0[sl], tr = T0[sr];
+      auto upd = [&](float l, float c, float rr, float d, float u, float b, float n) {
+        const float nb = ((l + rr) + (d + u)) + (b + n);
+        return fmaf(k, fmaf(-6.0f, c, nb), c);
+      };
+      float4 v;
+      v.x = upd(tl, t.x, last == 0 ? tr : t.y, td.x, tu.x, tb.x, tn.x);
+      v.y = upd(t.x, t.y, last == 1 ? tr : t.z, td.y, tu.y, tb.y, tn.y);
+      v.z = upd(t.y, t.z, last == 2 ? tr : t.w, td.z, tu.z, tb.z, tn.z);
+      v.w = upd(t.z, t.w, tr, td.w, tu.w, tb.w, tn.w);
+      if (act) *reinterpret_cast<float4*>(op) = v;
+      op += sz;
+      tb = t;
+      t = tn;
+      ce = cs;
+      cs = cn;
+      if (++cn == PB_NS) {
+        cn = 0;
+        phase ^= 1u;
       }
     }
     __syncthreads();  // every copy of the item has landed and been read: the barriers start over
