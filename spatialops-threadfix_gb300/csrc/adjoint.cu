@@ -235,12 +235,12 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
   {
     const double* t0 = T + (long)sz * z0;
     const double* a0 = Ain + (long)sz * z0;
-    const double tc = __ldg(t0 + ic);
-    ac = __ldg(a0 + ic);
-    tn = __ldg(t0 + sz + ic);
-    an = __ldg(a0 + sz + ic);
-    dazl = ac - __ldg(a0 - sz + ic);
-    dtzl = tc - __ldg(t0 - sz + ic);
+    const double tc = ld_step(t0 + ic);
+    ac = ld_step(a0 + ic);
+    tn = ld_step(t0 + sz + ic);
+    an = ld_step(a0 + sz + ic);
+    dazl = ac - ld_step(a0 - sz + ic);
+    dtzl = tc - ld_step(t0 - sz + ic);
     dazh = an - ac;
     dtzh = tn - tc;
     const int b = z0 & 1;
@@ -248,16 +248,16 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
     X = stage(b ^ 1, 0, si, tn);
     Y = stage(b ^ 1, 1, si, an);
     if (halo) {
-      stage(b, 0, hi, __ldg(t0 + ih));
-      stage(b, 1, hi, __ldg(a0 + ih));
-      stage(b ^ 1, 0, hi, __ldg(t0 + sz + ih));
-      stage(b ^ 1, 1, hi, __ldg(a0 + sz + ih));
+      stage(b, 0, hi, ld_step(t0 + ih));
+      stage(b, 1, hi, ld_step(a0 + ih));
+      stage(b ^ 1, 0, hi, ld_step(t0 + sz + ih));
+      stage(b ^ 1, 1, hi, ld_step(a0 + sz + ih));
     }
     __syncthreads();
     faces(b, X0, Y0);
     const long o2 = (long)sz * min(z0 + 2, nz);
-    tn2 = __ldg(T + o2 + ic);
-    an2 = __ldg(Ain + o2 + ic);
+    tn2 = ld_step(T + o2 + ic);
+    an2 = ld_step(Ain + o2 + ic);
   }
   const bool active = x0 + tx < nx && y0 + ty < ny;
   auto chain = [&](double kxl, double kxh, double kyl, double kyh, double kzl, double kzh, double daxh, double dayh) {
@@ -300,9 +300,9 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
     const long o = (long)sz * z + ic;
     const double daxh = sm.ax[buf][ty][tx + 1], dayh = sm.ay[buf][ty + 1][tx];
     const double dtxh = sm.tx[buf][ty][tx + 1], dtyh = sm.ty[buf][ty + 1][tx];
-    const double kzh = __ldg(lfz + o + sz), kzl = __ldg(lfz + o), kyh = __ldg(lfy + o + sy), kyl = __ldg(lfy + o),
-                 kxh = __ldg(lfx + o + 1), kxl = __ldg(lfx + o);
-    const double g = active ? glam[o] : 0.0;
+    const double kzh = ld_step(lfz + o + sz), kzl = ld_step(lfz + o), kyh = ld_step(lfy + o + sy), kyl = ld_step(lfy + o),
+                 kxh = ld_step(lfx + o + 1), kxl = ld_step(lfx + o);
+    const double g = active ? ld_step(glam + o) : 0.0;
     const double v = fma(hdt, chain(kxl, kxh, kyl, kyh, kzl, kzh, daxh, dayh), ac);
     const double gn = fma(-hdt, products(daxh, dayh, dtxh, dtyh), g);
     const bool more = z + 1 < z1;
@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
       X = stage(buf, 0, si, tn2);
       Y = stage(buf, 1, si, an2);
       if (halo) {
-        stage(buf, 0, hi, __ldg(T + (long)sz * (z + 2) + ih));
-        stage(buf, 1, hi, __ldg(Ain + (long)sz * (z + 2) + ih));
+        stage(buf, 0, hi, ld_step(T + (long)sz * (z + 2) + ih));
+        stage(buf, 1, hi, ld_step(Ain + (long)sz * (z + 2) + ih));
       }
     }
     if (!more) step_end();
@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_adjoint_soft_kernel(
     tn = tn2;
     an = an2;
     const long o3 = (long)sz * min(z + 3, nz);  // past nz: read again, not used
-    tn2 = __ldg(T + o3 + ic);
-    an2 = __ldg(Ain + o3 + ic);
+    tn2 = ld_step(T + o3 + ic);
+    an2 = ld_step(Ain + o3 + ic);
   }
 }
 

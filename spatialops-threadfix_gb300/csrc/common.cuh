@@ -140,6 +140,25 @@ inline void launch_step_kernel(void (*kern)(Params...), dim3 grid, dim3 block, s
   cudaLaunchKernelEx(&c, kern, Params(args)...);  // an error is found by the caller's launch check
 }
 __device__ __forceinline__ void step_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Every load a step kernel makes of what an earlier kernel wrote: an ordinary load that stays after
+// step_begin.  __ldg, and loads through const __restrict__ pointers, promise memory that no kernel
+// changes; the compiler may move them above the wait, and then the first planes of a block's chunk
+// are read while the kernel before still writes them.
+__device__ __forceinline__ double ld_step(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_step(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 ld_step(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ void step_end() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // SM count of the current device, queried once (callers on several threads may race to the

@@ -112,18 +112,18 @@ __global__ void __launch_bounds__(BX* BY) heat_step_kernel(const T* __restrict__
   auto at = [&](int i, int j, int k) { return (long)i + (long)sy * j + sz * k; };
 
   step_begin();
-  T tc = __ldg(tin + at(xc, yc, z0));
-  T lc = __ldg(lam + at(xc, yc, z0));
-  T fzlo = face_flux<T, A, MODE>(__ldg(lam + at(xc, yc, z0 - 1)), lc, __ldg(tin + at(xc, yc, z0 - 1)), tc, p.c0[2],
+  T tc = ld_step(tin + at(xc, yc, z0));
+  T lc = ld_step(lam + at(xc, yc, z0));
+  T fzlo = face_flux<T, A, MODE>(ld_step(lam + at(xc, yc, z0 - 1)), lc, ld_step(tin + at(xc, yc, z0 - 1)), tc, p.c0[2],
                                  p.c1[2]);
   for (int z = z0; z < z1; ++z) {
     const int buf = z & 1;
-    const T tn = __ldg(tin + at(xc, yc, z + 1));
-    const T ln = __ldg(lam + at(xc, yc, z + 1));
+    const T tn = ld_step(tin + at(xc, yc, z + 1));
+    const T ln = ld_step(lam + at(xc, yc, z + 1));
     const T fzhi = face_flux<T, A, MODE>(lc, ln, tc, tn, p.c0[2], p.c1[2]);
-    const T fx = face_flux<T, A, MODE>(__ldg(lam + at(xc - 1, yc, z)), lc, __ldg(tin + at(xc - 1, yc, z)), tc, p.c0[0],
+    const T fx = face_flux<T, A, MODE>(ld_step(lam + at(xc - 1, yc, z)), lc, ld_step(tin + at(xc - 1, yc, z)), tc, p.c0[0],
                                        p.c1[0]);
-    const T fy = face_flux<T, A, MODE>(__ldg(lam + at(xc, yc - 1, z)), lc, __ldg(tin + at(xc, yc - 1, z)), tc, p.c0[1],
+    const T fy = face_flux<T, A, MODE>(ld_step(lam + at(xc, yc - 1, z)), lc, ld_step(tin + at(xc, yc - 1, z)), tc, p.c0[1],
                                        p.c1[1]);
     sfx[buf][ty][tx] = fx;
     sfy[buf][ty][tx] = fy;
@@ -131,16 +131,16 @@ __global__ void __launch_bounds__(BX* BY) heat_step_kernel(const T* __restrict__
       // +y halo face of column x: between rows y0+BY-1 and y0+BY
       const int yh = y0 + BY;
       if (yh <= ny && x <= nx) {
-        sfy[buf][BY][tx] = face_flux<T, A, MODE>(__ldg(lam + at(xc, yh - 1, z)), __ldg(lam + at(xc, yh, z)),
-                                                 __ldg(tin + at(xc, yh - 1, z)), __ldg(tin + at(xc, yh, z)), p.c0[1],
+        sfy[buf][BY][tx] = face_flux<T, A, MODE>(ld_step(lam + at(xc, yh - 1, z)), ld_step(lam + at(xc, yh, z)),
+                                                 ld_step(tin + at(xc, yh - 1, z)), ld_step(tin + at(xc, yh, z)), p.c0[1],
                                                  p.c1[1]);
       }
     } else if (ty == 1 && tx < BY) {
       // +x halo face of row y0+tx: between columns x0+BX-1 and x0+BX
       const int xh = x0 + BX, yr = y0 + tx;
       if (xh <= nx && yr < ny) {
-        sfx[buf][tx][BX] = face_flux<T, A, MODE>(__ldg(lam + at(xh - 1, yr, z)), __ldg(lam + at(xh, yr, z)),
-                                                 __ldg(tin + at(xh - 1, yr, z)), __ldg(tin + at(xh, yr, z)), p.c0[0],
+        sfx[buf][tx][BX] = face_flux<T, A, MODE>(ld_step(lam + at(xh - 1, yr, z)), ld_step(lam + at(xh, yr, z)),
+                                                 ld_step(tin + at(xh - 1, yr, z)), ld_step(tin + at(xh, yr, z)), p.c0[0],
                                                  p.c1[0]);
       }
     }
@@ -1219,7 +1219,7 @@ __global__ void __maxnreg__(40)
     const long m = first + sz * (z0 - 1) + xc + 1 + (long)gx * min(k + 1, nr + 1);
     t[k] = lds(T0 + (k + 1) * g4 + 4);
     l[k] = lds(L0 + (k + 1) * g4 + 4);
-    fz[k] = (__ldg(ldata + m) + l[k]) * (t[k] - __ldg(tdata + m));
+    fz[k] = (ld_step(ldata + m) + l[k]) * (t[k] - ld_step(tdata + m));
   }
   float* out = tout + (long)x + (long)gx * y0 + sz * z0;
   int st = 0, ph = 0;  // stage of plane z, phase parity of plane z + 1's stage

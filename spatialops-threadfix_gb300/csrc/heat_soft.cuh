@@ -105,12 +105,12 @@ __global__ void __launch_bounds__(HS_X* HS_Y, UNIT ? 4 : 3) heat_soft_kernel(
   auto load = [&](int z) {
     Coef k;
     const long o = (long)sz * z;
-    k.x = __ldg(lfx + o + ic);
-    k.y = __ldg(lfy + o + ic);
-    k.z = __ldg(lfz + o + sz + ic);  // plane z + 1 <= nz
+    k.x = ld_step(lfx + o + ic);
+    k.y = ld_step(lfy + o + ic);
+    k.z = ld_step(lfz + o + sz + ic);  // plane z + 1 <= nz
     k.e = 0.0;
     if (xface) {
-      k.e = ty == 0 ? __ldg(lfy + o + xc + sy * (y0 + HS_Y)) : __ldg(lfx + o + x0 + HS_X + sy * (y0 + tx));
+      k.e = ty == 0 ? ld_step(lfy + o + xc + sy * (y0 + HS_Y)) : ld_step(lfx + o + x0 + HS_X + sy * (y0 + tx));
     }
     return k;
   };
@@ -133,18 +133,18 @@ __global__ void __launch_bounds__(HS_X* HS_Y, UNIT ? 4 : 3) heat_soft_kernel(
   Coef k = load(z0);
   {
     const double* t0 = tin + (long)sz * z0;
-    tc = __ldg(t0 + ic);
-    tn = __ldg(t0 + sz + ic);
-    const double tm = __ldg(t0 - sz + ic);
-    fzlo = __dmul_rn(__ldg(lfz + (long)sz * z0 + ic), __dsub_rn(scaled(tc, 2), scaled(tm, 2)));
+    tc = ld_step(t0 + ic);
+    tn = ld_step(t0 + sz + ic);
+    const double tm = ld_step(t0 - sz + ic);
+    fzlo = __dmul_rn(ld_step(lfz + (long)sz * z0 + ic), __dsub_rn(scaled(tc, 2), scaled(tm, 2)));
     const int b = z0 & 1;
     const SoftVal X0 = stage(b, si, tc);
     X = stage(b ^ 1, si, tn);
     if (SOFTZ) Z = softfp::unpack(scaled(tn, 2));
     if (halo) {
       const int2 h = halo_at();
-      stage(b, h.y, __ldg(t0 + h.x));
-      stage(b ^ 1, h.y, __ldg(t0 + sz + h.x));
+      stage(b, h.y, ld_step(t0 + h.x));
+      stage(b ^ 1, h.y, ld_step(t0 + sz + h.x));
     }
     __syncthreads();
     fzhi = __dmul_rn(k.z, __dsub_rn(scaled(tn, 2), scaled(tc, 2)));
@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(HS_X* HS_Y, UNIT ? 4 : 3) heat_soft_kernel(
     sfy[b][ty][tx] = fy;
     extra(b, k.e);
     const long o2 = (long)sz * min(z0 + 2, nz);
-    tn2 = __ldg(tin + o2 + ic);
-    if (!UNIT) hn = halo ? __ldg(tin + o2 + halo_at().x) : 0.0;
+    tn2 = ld_step(tin + o2 + ic);
+    if (!UNIT) hn = halo ? ld_step(tin + o2 + halo_at().x) : 0.0;
     if (z0 + 1 < z1) k = load(z0 + 1);
   }
   auto store = [&](int z, double v) {
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(HS_X* HS_Y, UNIT ? 4 : 3) heat_soft_kernel(
     const SoftVal Xn = stage(buf, si, tn2);
     if (halo) {
       const int2 h = halo_at();
-      stage(buf, h.y, UNIT ? __ldg(tin + (long)sz * (z + 2) + h.x) : hn);
+      stage(buf, h.y, UNIT ? ld_step(tin + (long)sz * (z + 2) + h.x) : hn);
     }
     const double prod = __dmul_rn(p.hdt, sum);
     double gz;
@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(HS_X* HS_Y, UNIT ? 4 : 3) heat_soft_kernel(
     const long o3 = (long)sz * min(z + 3, nz);
     tc = tn;
     tn = tn2;
-    tn2 = __ldg(tin + o3 + ic);
-    if (!UNIT) hn = halo ? __ldg(tin + o3 + halo_at().x) : 0.0;
+    tn2 = ld_step(tin + o3 + ic);
+    if (!UNIT) hn = halo ? ld_step(tin + o3 + halo_at().x) : 0.0;
     k = load(min(z + 2, z1 - 1));
     store(z, v);
     fy = gy;

@@ -275,9 +275,9 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared& sm, const doubl
   SoftVal X;  // of plane z + 1
   {
     const double* t0 = tin + (long)sz * z0;
-    tc = __ldg(t0 + ic);
-    tn = __ldg(t0 + sz + ic);
-    const double tm = __ldg(t0 - sz + ic);
+    tc = ld_step(t0 + ic);
+    tn = ld_step(t0 + sz + ic);
+    const double tm = ld_step(t0 - sz + ic);
     fzlo = __dmul_rn(s, __dsub_rn(tc, tm));
     fzhi = __dmul_rn(s, __dsub_rn(tn, tc));
     const int b = z0 & 1;
@@ -285,8 +285,8 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared& sm, const doubl
     X = stage(b ^ 1, si, tn);
     if (halo) {
       const int2 c = sm.halo[h];
-      stage(b, c.y, __ldg(t0 + c.x));
-      stage(b ^ 1, c.y, __ldg(t0 + sz + c.x));
+      stage(b, c.y, ld_step(t0 + c.x));
+      stage(b ^ 1, c.y, ld_step(t0 + sz + c.x));
     }
     __syncthreads();
     bool ok;
@@ -299,7 +299,7 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared& sm, const doubl
     sm.fx[b][fi] = fx;
     sm.fy[b][gi] = fy;
     extra(b);
-    tn2 = __ldg(tin + (long)sz * min(z0 + 2, nz) + ic);
+    tn2 = ld_step(tin + (long)sz * min(z0 + 2, nz) + ic);
   }
   const bool active = in_tile && x0 + tx < nx && y0 + ty < ny;
   const bool edge = x0 + tx == 0 || x0 + tx == nx - 1 || y0 + ty == 0 || y0 + ty == ny - 1;
@@ -333,7 +333,7 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared& sm, const doubl
     const SoftVal Xn = stage(buf, si, tn2);
     if (halo) {
       const int2 c = sm.halo[h];
-      stage(buf, c.y, __ldg(tin + (long)sz * (z + 2) + c.x));
+      stage(buf, c.y, ld_step(tin + (long)sz * (z + 2) + c.x));
     }
     const double prod = __dmul_rn(hdt, sum);
     const double gz = __dmul_rn(s, dz);
@@ -347,7 +347,7 @@ __device__ __forceinline__ void patch_soft_item(PatchSoftShared& sm, const doubl
     extra(nb);
     tc = tn;
     tn = tn2;
-    tn2 = __ldg(tin + (long)sz * min(z + 3, P.nz) + ic);  // past nz: read again, not used
+    tn2 = ld_step(tin + (long)sz * min(z + 3, P.nz) + ic);  // past nz: read again, not used
     store(z, v);
     fx = gx;
     fy = gy;

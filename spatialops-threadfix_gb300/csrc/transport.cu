@@ -53,10 +53,10 @@ struct TrArgs {
 template <typename T>
 __device__ __forceinline__ T face_flux(const TrArgs<T>& a, long f, long s, const T* vel) {
   const T* p = a.phi;
-  const T il = (__ldg(a.lam + f - s) + __ldg(a.lam + f)) * T(0.5);
-  const T g4 = ((__ldg(p + f - 2 * s) * a.q0 + __ldg(p + f - s) * a.q1) + __ldg(p + f) * a.q2) + __ldg(p + f + s) * a.q3;
-  const T uf = __ldg(vel + f);
-  const T up = (uf > T(0)) ? __ldg(p + f - s) : __ldg(p + f);
+  const T il = (ld_step(a.lam + f - s) + ld_step(a.lam + f)) * T(0.5);
+  const T g4 = ((ld_step(p + f - 2 * s) * a.q0 + ld_step(p + f - s) * a.q1) + ld_step(p + f) * a.q2) + ld_step(p + f + s) * a.q3;
+  const T uf = ld_step(vel + f);
+  const T up = (uf > T(0)) ? ld_step(p + f - s) : ld_step(p + f);
   return a.nu * il * g4 - uf * up;
 }
 
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
   const int xc = min(x, n), yc = min(y, n);  // column/row n is a ghost: valid memory
   auto positive = [](double u) { return __double_as_longlong(u) > 0; };
   auto coef = [&](const double* kf, long f, long s) {
-    return KF ? __ldg(kf + f) : kc * (__ldg(a.lam + f - s) + __ldg(a.lam + f));
+    return KF ? ld_step(kf + f) : kc * (ld_step(a.lam + f - s) + ld_step(a.lam + f));
   };
   auto flux = [&](double k, double u, double pm2, double pm1, double p0, double pp1) {
     const double g = fma(27.0, p0 - pm1, pm2 - pp1);
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
   };
   auto flux_at = [&](const double* kf, const double* vel, long f, long s) {
     const double* p = a.phi + f;
-    return flux(coef(kf, f, s), __ldg(vel + f), __ldg(p - 2 * s), __ldg(p - s), __ldg(p), __ldg(p + s));
+    return flux(coef(kf, f, s), ld_step(vel + f), ld_step(p - 2 * s), ld_step(p - s), ld_step(p), ld_step(p + s));
   };
   // the extra faces: warp 0 those above the tile, lanes 0..7 of warp 1 those right of it
   const bool xface = (ty == 0 && y0 + TY <= n && x <= n) || (ty == 1 && tx < TY && x0 + TX <= n && y0 + tx < n);
@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
   const long ce = ty == 0 ? (long)xc + (long)sy * (y0 + TY) : (long)(x0 + TX) + (long)sy * (y0 + tx);
   step_begin();
   long c = c0 + sz * z0;
-  double pm1 = __ldg(a.phi + c - sz), p0 = __ldg(a.phi + c), p1 = __ldg(a.phi + c + sz);
-  double fzlo = flux(coef(kfz, c, sz), __ldg(a.w + c), __ldg(a.phi + c - 2 * sz), pm1, p0, p1);
+  double pm1 = ld_step(a.phi + c - sz), p0 = ld_step(a.phi + c), p1 = ld_step(a.phi + c + sz);
+  double fzlo = flux(coef(kfz, c, sz), ld_step(a.w + c), ld_step(a.phi + c - 2 * sz), pm1, p0, p1);
 #pragma unroll 1
   for (int z = z0; z < z1; ++z, c += sz) {
     const int buf = z & 1;
@@ -225,12 +225,12 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
         if (SECOND) prefetch_l2(a.base + cp);
       }
     }
-    const double p2 = __ldg(a.phi + c + 2 * sz);
-    const double base = SECOND ? a.base[c] : 0.0;
-    const double fx = flux(coef(kfx, c, 1), __ldg(a.u + c), __ldg(a.phi + c - 2), __ldg(a.phi + c - 1), p0,
-                           __ldg(a.phi + c + 1));
-    const double fy = flux(coef(kfy, c, sy), __ldg(a.v + c), __ldg(a.phi + c - 2 * sy), __ldg(a.phi + c - sy), p0,
-                           __ldg(a.phi + c + sy));
+    const double p2 = ld_step(a.phi + c + 2 * sz);
+    const double base = SECOND ? ld_step(a.base + c) : 0.0;
+    const double fx = flux(coef(kfx, c, 1), ld_step(a.u + c), ld_step(a.phi + c - 2), ld_step(a.phi + c - 1), p0,
+                           ld_step(a.phi + c + 1));
+    const double fy = flux(coef(kfy, c, sy), ld_step(a.v + c), ld_step(a.phi + c - 2 * sy), ld_step(a.phi + c - sy), p0,
+                           ld_step(a.phi + c + sy));
     sfx[buf][ty][tx] = fx;
     sfy[buf][ty][tx] = fy;
     if (xface) {
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
       else
         sfx[buf][tx][TX] = flux_at(kfx, a.u, f, 1);
     }
-    const double fzhi = flux(coef(kfz, c + sz, sz), __ldg(a.w + c + sz), pm1, p0, p1, p2);
+    const double fzhi = flux(coef(kfz, c + sz, sz), ld_step(a.w + c + sz), pm1, p0, p1, p2);
     const double dz = fzhi - fzlo;
     __syncthreads();
     if (z + 1 == z1) step_end();
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_f32_staged_kernel(TrAr
   auto at = [&](int i, int j, int k) { return (long)i + (long)sy * j + sz * k; };
   // the column's phi window and the low z face of plane z0, from global memory
   const long c0 = at(xc, yc, z0);
-  float pm1 = __ldg(a.phi + c0 - sz), p0 = __ldg(a.phi + c0), p1 = __ldg(a.phi + c0 + sz);
+  float pm1 = ld_step(a.phi + c0 - sz), p0 = ld_step(a.phi + c0), p1 = ld_step(a.phi + c0 + sz);
   float fzlo = face_flux(a, c0, sz, a.w);
   const int ci = (ty + G) * SPW + tx + G;
   // this column's global values of plane z (velocities on its faces, the FP64 state), loaded one
@@ -369,11 +369,11 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_f32_staged_kernel(TrAr
   auto load_col = [&](int z) {
     Col q;
     const long c = at(xc, yc, z);
-    q.ul = __ldg(a.u + c);
-    q.uh = __ldg(a.u + c + 1);
-    q.vl = __ldg(a.v + c);
-    q.vh = __ldg(a.v + c + sy);
-    q.wh = __ldg(a.w + c + sz);
+    q.ul = ld_step(a.u + c);
+    q.uh = ld_step(a.u + c + 1);
+    q.vl = ld_step(a.v + c);
+    q.vh = ld_step(a.v + c + sy);
+    q.wh = ld_step(a.w + c + sz);
     q.acc = a.acc[c];
     q.base = SECOND ? a.base[c] : 0.0;
     return q;
@@ -458,7 +458,7 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 }
 
 __device__ __forceinline__ float2 tsub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-__device__ __forceinline__ float2 tld2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+__device__ __forceinline__ float2 tld2(const float* p) { return ld_step(reinterpret_cast<const float2*>(p)); }
 __device__ __forceinline__ float2 tsh2(const float* p) { return *reinterpret_cast<const float2*>(p); }
 
 // sflux for two faces at once (same operand order).
@@ -567,14 +567,14 @@ __global__ void __launch_bounds__(PTX* TY) transport_stage_f32_pair_kernel(TrArg
     Col q;
     const long c = at(xc, yc, z);
     q.ul = tld2(a.u + c);  // faces x-1/2, x+1/2
-    q.u2 = __ldg(a.u + c + 2);  // face x+3/2
+    q.u2 = ld_step(a.u + c + 2);  // face x+3/2
     q.vl = tld2(a.v + c);
     q.vh = tld2(a.v + c + sy);
     q.wh = tld2(a.w + c + sz);
-    q.acc0 = a.acc[c];
-    q.acc1 = a.acc[c + 1];
-    q.base0 = SECOND ? a.base[c] : 0.0;
-    q.base1 = SECOND ? a.base[c + 1] : 0.0;
+    q.acc0 = ld_step(a.acc + c);
+    q.acc1 = ld_step(a.acc + c + 1);
+    q.base0 = SECOND ? ld_step(a.base + c) : 0.0;
+    q.base1 = SECOND ? ld_step(a.base + c + 1) : 0.0;
     return q;
   };
   const float2 NU = make_float2(a.nu, a.nu), Q0 = make_float2(a.q0, a.q0), Q1 = make_float2(a.q1, a.q1),
