@@ -145,7 +145,12 @@ int nebo_heat_step(const nebo_field* T, const nebo_field* Tout, const nebo_field
                    const double spacing[3], nebo_stream_t stream);
 
 /* steps Euler steps, ping-ponging T and Ttmp; the result is left in T (ghosts filled).
- * use_graph != 0 captures the step sequence in a CUDA graph once and replays it. */
+ * use_graph != 0 captures the step sequence in a CUDA graph once and replays it.
+ * FP64 runs of three or more steps (two in general spacing) form lambda's face coefficients once,
+ * in scratch of three fields from the stream-ordered pool (given back at the end of the run; a
+ * cached graph keeps up to 1 GiB of it, larger fields are launched step by step instead).  Where
+ * that memory is not to be had, and while the caller records a graph, every step forms them.  The
+ * bits are the same. */
 int nebo_heat_run(const nebo_field* T, const nebo_field* Ttmp, const nebo_field* lam, int steps,
                   double dt, const double spacing[3], int use_graph, nebo_stream_t stream);
 
@@ -229,7 +234,8 @@ int nebo_fastmath_eval(int fn, const double* x, double* y, size_t n, nebo_stream
  *             call after loading the FP64 arena.
  *   sync:     after run, make the FP64 arena `which` hold the state (FP32: widened, FP32X2:
  *             hi + lo).
- *   autotune: times tile widths 16/32/64 per x-extent class and keeps the fastest; in NEBO_F32
+ *   autotune: times tile widths 16/32/64 per x-extent class and keeps the fastest (FP64 tiles are
+ *             fitted to each patch, at most that wide); in NEBO_F32
  *             mode (row strips of up to 1024 cells, no tile width) it picks the z extent of the
  *             work items instead (whole patch, 32 or 16 planes).  Clobbers the arenas: call it
  *             before loading data.
@@ -262,7 +268,10 @@ int nebo_patchset_run(nebo_patchset* ps, int start, int steps, int use_graph, in
  * Each RK stage is one kernel.  FP32 with n even: staged planes (8-byte copies), and with every
  * float field 8-byte aligned two cells per thread in packed FP32x2 arithmetic; odd n or
  * unaligned fields take a one-cell kernel (same results within FP32 rounding).  The coefficient
- * ghost fills and the FP32 copy of the state are made once per call: run many steps per call. */
+ * ghost fills and the FP32 copy of the state are made once per call: run many steps per call.
+ * FP64 runs of two or more steps form the face coefficients once, in scratch of three more fields
+ * from the stream-ordered pool (given back at the end of the call); where it is not to be had, and
+ * while the caller records a graph, every stage forms them.  The bits are the same. */
 size_t nebo_transport_work_bytes(int n, int dtype);
 int nebo_transport_run(double* phi, const void* u, const void* v, const void* w, const void* lam,
                        int n, int steps, double dt, double nu, int dtype, void* work,

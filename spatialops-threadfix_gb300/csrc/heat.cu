@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(BX* BY) heat_step_kernel(const T* __restrict__
 }
 
 
-// FP32 heat step with an asynchronous plane pipeline.  FP32 arithmetic is nearly free on this
+// FP32 heat step with an asynchronous plane pipeline, for rows of more than SL_MAXX cells (narrower
+// ones run on bulk-copied slabs, below).  FP32 arithmetic is nearly free on this
 // GPU, so the kernel is bound by instruction issue and by the bytes it keeps in flight: each block
 // streams planes of T and lambda (its 32x32 tile plus a one-cell halo) into a ring of NS shared-
 // memory stages with cp.async, using no registers for the loads in flight, and each thread owns a
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_step_f32_async_kernel(const fl
   cp_async_wait<0>();
 }
 
-// FP32 heat step on packed pairs (the 8-byte-aligned case).  Each thread owns two x-adjacent
+// FP32 heat step on packed pairs (rows of more than SL_MAXX cells, 8-byte aligned).  Each thread owns two x-adjacent
 // cells in two rows (a 2 x 2 block; 256 threads cover the same 32 x 32 tile and the same ring
 // of NS stages as heat_step_f32_async_kernel).  The cells x, x+1 (x even) and their x
 // neighbours x-1, x+2 are the two aligned pairs A = (x-1, x) and B = (x+1, x+2) of the stage

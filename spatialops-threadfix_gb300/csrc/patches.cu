@@ -9,8 +9,9 @@
 //     or FP32 states (half the bytes), or two-float states (FP32 arithmetic, ~48-bit state);
 //   * a work list enumerates (patch, x-tile, y-tile, z-chunk) items; a fixed grid of blocks
 //     (a multiple of the SM count) strides through it, so small and large patches share SMs;
-//   * tiles are TX x TY = 256 cells per plane with TX in {16, 32, 64} per patch (the autotuner
-//     times each candidate on the patches of each x-extent class and keeps the fastest);
+//   * FP64 tiles hold up to 256 cells of a plane, fitted to the patch's extents (tile_shape) under a
+//     width limit of 16, 32 or 64 per patch (the autotuner times each on the patches of each
+//     x-extent class and keeps the fastest); FP32 items are strips of full rows;
 //   * each item is the fused heat step of nebo_heat_step: face fluxes computed once, high
 //     faces shared through shared memory, z-face carried in a register, and the new values
 //     written to the interior and to their periodic ghost images in the same pass.
