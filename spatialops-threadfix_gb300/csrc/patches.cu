@@ -684,11 +684,12 @@ __global__ void __launch_bounds__(PT_THREADS) patches_f32_bulk_kernel(const Patc
 }
 
 // FP64 windows -> FP32 slab layout (interiors only) and back (whole windows: each cell of a
-// window takes its periodic interior source, so the ghosts are filled in the same pass).  A warp
-// takes a row (unpacking two), four of its cells per lane in flight; values widen and round by their
-// bits (a hardware conversion issues on the FP64 pipe).  Bound by the 8-byte stores: 512 patches of
-// 16..96 cells an edge back to windows 623 -> 357 us (an index division per cell before), 207 of it
-// the stores alone.
+// window takes its periodic interior source, so the ghosts are filled in the same pass).  Packing, a warp takes a row, four of its cells per lane in flight.  Unpacking, a thread
+// takes four consecutive window elements whatever rows they fall in: windows start on 256-byte
+// boundaries, so the results are two 16-byte stores on a whole sector.  Values widen and round by
+// their bits (a hardware conversion issues on the FP64 pipe).  512 patches of 16..96 cells an edge
+// back to windows (1.2 GB): an index division per cell 623 us, a warp per row with 8-byte stores 358,
+// two elements a thread 348, four 287 (4.2 TB/s).
 __device__ __forceinline__ float narrow(double v) {  // rounded to nearest, subnormal floats included
   const int e = fixmath::dexp(v);
   return e <= 896 && e >= 872 ? (float)v : fixmath::f64_to_f32_rn(v);
@@ -721,36 +722,37 @@ __global__ void __launch_bounds__(256) patches_pack_f32_kernel(const PatchDev* _
 __global__ void __launch_bounds__(256) patches_unpack_f32_kernel(const PatchDev* __restrict__ patches, int npatch,
                                                                  const float* __restrict__ a32,
                                                                  double* __restrict__ a64) {
-  const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
   for (int p = blockIdx.y; p < npatch; p += gridDim.y) {
     const PatchDev P = patches[p];
     const int nx = P.nx, ny = P.ny, nz = P.nz, gx = nx + 2, gy = ny + 2;
-    const long rows = (long)gy * (nz + 2);
-    // two rows at a time: eight loads in flight per lane
-    for (long r = 2 * (blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5)); r < rows; r += 2 * nw) {
-      const float* from[2];
-      double* to[2];
-      int w[2];
+    const long total = (long)gx * gy * (nz + 2), step = 4 * (long)gridDim.x * blockDim.x;
+    double* to = a64 + P.offset;
+    for (long q = 4 * (blockIdx.x * (long)blockDim.x + threadIdx.x); q < total; q += step) {
+      const long r = fast_div(q, gx);
+      int c = (int)(q - r * gx), z = (int)fast_div(r, gy), y = (int)(r - (long)z * gy);
+      const float* from = a32 + P.off32 + ((long)wrap1(z - 1, nz) * ny + wrap1(y - 1, ny)) * P.pitch32;
+      float v[4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const long q = min(r + h, rows - 1);
-        const int z = (int)fast_div(q, gy), y = (int)(q - (long)z * gy);
-        from[h] = a32 + P.off32 + ((long)wrap1(z - 1, nz) * ny + wrap1(y - 1, ny)) * P.pitch32;
-        to[h] = a64 + P.offset + q * gx;
-        w[h] = r + h < rows ? gx : 0;
+      for (int k = 0; k < 4; ++k) {
+        v[k] = q + k < total ? __ldg(from + wrap1(c - 1, nx)) : 0.0f;
+        if (++c == gx) {  // the next window row (past the window's end none is read)
+          c = 0;
+          if (++y == gy) {
+            y = 0;
+            ++z;
+          }
+          from = a32 + P.off32 + ((long)wrap1(min(z, nz + 1) - 1, nz) * ny + wrap1(y - 1, ny)) * P.pitch32;
+        }
       }
-      for (int x = lane; x < gx; x += 128) {
-        float v[8];
+      double w[4];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int c = x + 32 * (k & 3);
-          v[k] = c < w[k >> 2] ? __ldg(from[k >> 2] + wrap1(c - 1, nx)) : 0.0f;
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int c = x + 32 * (k & 3);
-          if (c < w[k >> 2]) to[k >> 2][c] = fixmath::f32_to_f64(v[k]);
-        }
+      for (int k = 0; k < 4; ++k) w[k] = fixmath::f32_to_f64(v[k]);
+      if (q + 3 < total) {
+        *reinterpret_cast<double2*>(to + q) = make_double2(w[0], w[1]);
+        *reinterpret_cast<double2*>(to + q + 2) = make_double2(w[2], w[3]);
+      } else {
+        for (int k = 0; k < 4; ++k)
+          if (q + k < total) to[q + k] = w[k];
       }
     }
   }
