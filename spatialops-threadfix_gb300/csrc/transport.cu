@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<float> a
 // low x and y faces come from each thread and the high ones through shared memory, the z face and
 // the column's phi window (z - 1 .. z + 2) stay in registers.  The halving of the second stage is an
 // exponent step.  What bounds it: the FP64 pipe at 23 operations per cell (40 in the form that sums
-// the four weighted values and compares u in FP64), 79 % busy: 188 -> 107 us per stage at 127^3.
+// the four weighted values and compares u in FP64), 79 % busy: 188 -> 110 us per stage at 127^3.
 // Error against 80-bit arithmetic after 20 steps: 1.15e-16 (2-norm), as before (1.16e-16).
 template <bool SECOND, bool KF>
 __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<double> a,
