@@ -18,7 +18,7 @@
 // one the reference's serial walk performs and the result is bit-identical.  FP64 with general
 // spacing evaluates the reference's own form (same operations, same order).  Both use _rn
 // intrinsics so no multiply-add is contracted.  FP32 (storage and arithmetic) uses the scaled
-// form with per-direction weights and lets the compiler fuse.
+// form with per-direction weights (its operations: face_f32 and what follows it).
 #include <climits>
 #include <map>
 #include <mutex>
@@ -170,6 +170,34 @@ __global__ void __launch_bounds__(BX* BY) heat_step_kernel(const T* __restrict__
 }
 
 
+// The arithmetic of the scalar FP32 steps, spelled out: a cell's bits then follow from its row pitch,
+// alignment and y alone, whichever kernel steps it and however the compiler would contract products
+// (FP32-forward gradients return doubles, in which a step's last FP32 bits show).  A face's flux is
+// s d; with X, Y, Z the differences (high - low) along the axes,
+//   T' = fma(w2, Z, fma(w1, Y, fma(w0, X, T))).
+// PAIRED (windows that heat_step_f32x2_kernel takes: even pitch, 8-byte aligned): its arithmetic,
+// every flux rounded.  Others: X takes the high flux unrounded, Y the low one in every fourth row
+// (y % 4 == 0).
+struct FaceF {
+  float s, d;  // la + lb, tb - ta
+};
+__device__ __forceinline__ FaceF face_f32(float la, float lb, float ta, float tb) {
+  return FaceF{__fadd_rn(la, lb), __fsub_rn(tb, ta)};
+}
+__device__ __forceinline__ float flux_f32(FaceF f) { return __fmul_rn(f.s, f.d); }
+template <bool PAIRED>
+__device__ __forceinline__ float x_diff_f32(FaceF lo, FaceF hi) {
+  return PAIRED ? __fsub_rn(flux_f32(hi), flux_f32(lo)) : fmaf(hi.s, hi.d, -flux_f32(lo));
+}
+// of a row y % 4 == 0 (elsewhere: the difference of the rounded fluxes)
+template <bool PAIRED>
+__device__ __forceinline__ float y_diff_f32(FaceF lo, float hi) {
+  return PAIRED ? __fsub_rn(hi, flux_f32(lo)) : fmaf(-lo.s, lo.d, hi);
+}
+__device__ __forceinline__ float update_f32(float t, float w0, float w1, float w2, float X, float Y, float Z) {
+  return fmaf(w2, Z, fmaf(w1, Y, fmaf(w0, X, t)));
+}
+
 // FP32 heat step with an asynchronous plane pipeline, for rows of more than SL_MAXX cells (narrower
 // ones run on bulk-copied slabs, below).  FP32 arithmetic is nearly free on this
 // GPU, so the kernel is bound by instruction issue and by the bytes it keeps in flight: each block
@@ -281,7 +309,7 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_step_f32_async_kernel(const fl
     for (int k = 0; k < CPT; ++k) {
       t[k] = sT[ci + k * HX];
       l[k] = sL[ci + k * HX];
-      fz[k] = (Lm[ci + k * HX] + l[k]) * (t[k] - Tm[ci + k * HX]);
+      fz[k] = flux_f32(face_f32(Lm[ci + k * HX], l[k], Tm[ci + k * HX], t[k]));
     }
   }
   float* out = tout + (long)x + (long)sy * yt + sz * z0;
@@ -299,24 +327,25 @@ __global__ void __launch_bounds__(BX* BY, 3) heat_step_f32_async_kernel(const fl
       const float* L0 = sL + i * PLANE;
       const float* Tn = sT + ((i + 1) % NS) * PLANE;
       const float* Ln = sL + ((i + 1) % NS) * PLANE;
-      float tn[CPT], ln[CPT], fy[CPT + 1];
+      float tn[CPT], ln[CPT], fy[CPT + 1];  // fy[k]: the face below cell k (k > 0)
 #pragma unroll
       for (int k = 0; k < CPT; ++k) {
         tn[k] = Tn[ci + k * HX];
         ln[k] = Ln[ci + k * HX];
       }
-      fy[0] = (L0[ci - HX] + l[0]) * (t[0] - T0[ci - HX]);
+      const FaceF below = face_f32(L0[ci - HX], l[0], T0[ci - HX], t[0]);
 #pragma unroll
-      for (int k = 1; k < CPT; ++k) fy[k] = (l[k - 1] + l[k]) * (t[k] - t[k - 1]);
-      fy[CPT] = (l[CPT - 1] + L0[ci + CPT * HX]) * (T0[ci + CPT * HX] - t[CPT - 1]);
+      for (int k = 1; k < CPT; ++k) fy[k] = flux_f32(face_f32(l[k - 1], l[k], t[k - 1], t[k]));
+      fy[CPT] = flux_f32(face_f32(l[CPT - 1], L0[ci + CPT * HX], t[CPT - 1], T0[ci + CPT * HX]));
       const bool zedge = z == 0 || z == nz - 1;
 #pragma unroll
       for (int k = 0; k < CPT; ++k) {
         const int c = ci + k * HX;
-        const float fxl = (L0[c - 1] + l[k]) * (t[k] - T0[c - 1]);
-        const float fxh = (l[k] + L0[c + 1]) * (T0[c + 1] - t[k]);
-        const float fzh = (l[k] + ln[k]) * (tn[k] - t[k]);
-        const float v = t[k] + w0 * (fxh - fxl) + w1 * (fy[k + 1] - fy[k]) + w2 * (fzh - fz[k]);
+        const float X = x_diff_f32<false>(face_f32(L0[c - 1], l[k], T0[c - 1], t[k]),
+                                          face_f32(l[k], L0[c + 1], t[k], T0[c + 1]));
+        const float Y = k == 0 ? y_diff_f32<false>(below, fy[1]) : __fsub_rn(fy[k + 1], fy[k]);
+        const float fzh = flux_f32(face_f32(l[k], ln[k], t[k], tn[k]));
+        const float v = update_f32(t[k], w0, w1, w2, X, Y, __fsub_rn(fzh, fz[k]));
         if (act[k]) {
           out[(long)sy * k] = v;
           if (edge[k] || zedge) store_images_only(tout, sy, sz, x, yt + k, z, nx, ny, nz, v);
@@ -1158,7 +1187,7 @@ __global__ void __launch_bounds__(BP_THREADS, 3) heat_step_f32_bulk2_kernel(cons
 // 40 registers let four blocks of 352 threads share an SM (64 registers, two blocks: 42.4 us).
 // At 323 x 197 x 150: 36.9 us = 3.1 TB/s, where 4-byte cp.async copies per cell took 108 us;
 // 322 x 198 x 150 (8-byte copies before) 69.8 -> 36.9, 401 x 301 x 201 141 -> 82.
-constexpr int SL_R = 4;        // rows per block
+constexpr int SL_R = 4;        // rows per block (the scalar arithmetic's row period)
 constexpr int SL_NS = 3;       // stages
 constexpr int SL_MAXX = 1024;  // threads per block
 
@@ -1166,6 +1195,7 @@ __host__ __device__ __forceinline__ uint32_t slab_stage_bytes(int gx) {  // byte
   return ((uint32_t)((SL_R + 2) * gx + 3) * 4u + 15u) & ~15u;
 }
 
+template <bool PAIRED>
 __global__ void __maxnreg__(40)
     heat_step_f32_slab_kernel(const float* __restrict__ tdata, float* __restrict__ tout,
                               const float* __restrict__ ldata, long total, int gx, long sz, int nx, int ny, int nz,
@@ -1222,7 +1252,7 @@ __global__ void __maxnreg__(40)
     const long m = first + sz * (z0 - 1) + xc + 1 + (long)gx * min(k + 1, nr + 1);
     t[k] = lds(T0 + (k + 1) * g4 + 4);
     l[k] = lds(L0 + (k + 1) * g4 + 4);
-    fz[k] = (ld_step(ldata + m) + l[k]) * (t[k] - ld_step(tdata + m));
+    fz[k] = flux_f32(face_f32(ld_step(ldata + m), l[k], ld_step(tdata + m), t[k]));
   }
   float* out = tout + (long)x + (long)gx * y0 + sz * z0;
   int st = 0, ph = 0;  // stage of plane z, phase parity of plane z + 1's stage
@@ -1239,7 +1269,8 @@ __global__ void __maxnreg__(40)
     const uint32_t sn0 = s0 + (uint32_t)sn * 2u * fb;
     uint32_t T1 = offT(z + 1, sn0), L1 = offL(z + 1, sn0);
     const uint32_t Tn = T1, Ln = L1;
-    float fy = (lds(L0 + 4) + l[0]) * (t[0] - lds(T0 + 4));
+    const FaceF below = face_f32(lds(L0 + 4), l[0], lds(T0 + 4), t[0]);
+    float fy = 0.0f;
     float v[SR];
 #pragma unroll
     for (int k = 0; k < SR; ++k) {
@@ -1248,14 +1279,14 @@ __global__ void __maxnreg__(40)
       T1 += g4;
       L1 += g4;
       const float tc = t[k], lc = l[k];
-      const float fxl = (lds(L0) + lc) * (tc - lds(T0));
-      const float fxh = (lc + lds(L0 + 8)) * (lds(T0 + 8) - tc);
+      const float X = x_diff_f32<PAIRED>(face_f32(lds(L0), lc, lds(T0), tc), face_f32(lc, lds(L0 + 8), tc, lds(T0 + 8)));
       const float tu = k + 1 < SR ? t[k + 1 < SR ? k + 1 : k] : lds(T0 + g4 + 4);
       const float lu = k + 1 < SR ? l[k + 1 < SR ? k + 1 : k] : lds(L0 + g4 + 4);
-      const float fyh = (lc + lu) * (tu - tc);
+      const float fyh = flux_f32(face_f32(lc, lu, tc, tu));
+      const float Y = k == 0 ? y_diff_f32<PAIRED>(below, fyh) : __fsub_rn(fyh, fy);
       const float tn = lds(T1 + 4), ln = lds(L1 + 4);
-      const float fzh = (lc + ln) * (tn - tc);
-      v[k] = fmaf(w2, fzh - fz[k], fmaf(w1, fyh - fy, fmaf(w0, fxh - fxl, tc)));
+      const float fzh = flux_f32(face_f32(lc, ln, tc, tn));
+      v[k] = update_f32(tc, w0, w1, w2, X, Y, __fsub_rn(fzh, fz[k]));
       fy = fyh;
       fz[k] = fzh;
       t[k] = tn;
@@ -1349,9 +1380,11 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
       NEBO_LAUNCH_CHECK("nebo_heat_step");
       return NEBO_OK;
     }
+    // every row of T and lambda starts 8-byte aligned (even pitch, aligned windows; nx is even then)
+    const bool vec = (vin.sy % 2 == 0) && ((uintptr_t)(vin.base - 1) % 8 == 0) && ((uintptr_t)(vl.base - 1) % 8 == 0);
     if (n[0] <= SL_MAXX) {
       const size_t smem = (size_t)SL_NS * 2 * slab_stage_bytes(gx) + SL_NS * sizeof(uint64_t);
-      auto kern = heat_step_f32_slab_kernel;
+      auto kern = vec ? heat_step_f32_slab_kernel<true> : heat_step_f32_slab_kernel<false>;
       NEBO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       const int bx = (n[0] + 31) / 32 * 32, yb = (n[1] + SL_R - 1) / SL_R;
       int bps = 0;
@@ -1369,9 +1402,7 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
       NEBO_LAUNCH_CHECK("nebo_heat_step");
       return NEBO_OK;
     }
-    // 8-byte copies when every row of T and lambda starts 8-byte aligned (even pitch, aligned
-    // windows); then nx is even too, which keeps the clamped column pairs aligned
-    const bool vec = (vin.sy % 2 == 0) && ((uintptr_t)(vin.base - 1) % 8 == 0) && ((uintptr_t)(vl.base - 1) % 8 == 0);
+    // vec: 8-byte copies, and the clamped column pairs stay aligned
     // one full wave: as many z chunks as the resident blocks allow (each chunk re-reads two
     // halo planes and fills the ring once, so more chunks than slots only cost)
     static std::atomic<int> per_sm[2];  // zero: not queried
