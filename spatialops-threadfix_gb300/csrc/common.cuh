@@ -176,13 +176,13 @@ inline int num_sms() {
   return n;
 }
 
-// Resident blocks per SM of `kernel` at `threads` threads and no dynamic shared memory, kept in
-// the caller's `cache` after the first query (same race rule as num_sms).
+// Resident blocks per SM of `kernel` at `threads` threads and `smem` bytes of dynamic shared memory,
+// kept in the caller's `cache` after the first query (same race rule as num_sms).
 template <class K>
-inline int blocks_per_sm(K kernel, int threads, std::atomic<int>& cache) {
+inline int blocks_per_sm(K kernel, int threads, std::atomic<int>& cache, size_t smem = 0) {
   int v = cache.load(std::memory_order_relaxed);
   if (!v) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, threads, 0) != cudaSuccess || v <= 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, threads, smem) != cudaSuccess || v <= 0) {
       cudaGetLastError();
       v = 1;
     }

@@ -1314,6 +1314,26 @@ __global__ void __maxnreg__(40)
   if (!ok) atomicAdd(&g_bulk_timeouts, 1u);
 }
 
+// Dynamic shared memory of the slab kernel for rows of nx cells (one ghost on either side).
+size_t slab_smem_bytes(int nx) { return (size_t)SL_NS * 2 * slab_stage_bytes(nx + 2) + SL_NS * sizeof(uint64_t); }
+
+// The slab kernels' shared memory exceeds the 48 KB default: the limit is raised once per device, to
+// the widest rows' bytes.  It belongs to the kernel, not to a launch: set to each launch's own bytes
+// it let a thread that steps narrow rows lower it under another's launch, which then failed.
+int slab_prepare() {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  NEBO_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 64 && (done.load() & (1ull << dev))) return NEBO_OK;
+  const int most = (int)slab_smem_bytes(SL_MAXX);
+  NEBO_CUDA_TRY(
+      cudaFuncSetAttribute(heat_step_f32_slab_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  NEBO_CUDA_TRY(
+      cudaFuncSetAttribute(heat_step_f32_slab_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  if (dev < 64) done.fetch_or(1ull << dev);
+  return NEBO_OK;
+}
+
 int check_heat(const nebo_field* T, const nebo_field* To, const nebo_field* L, const char* what) {
   int rc;
   if ((rc = check_field(T, what)) || (rc = check_field(To, what)) || (rc = check_field(L, what))) return rc;
@@ -1383,15 +1403,12 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
     // every row of T and lambda starts 8-byte aligned (even pitch, aligned windows; nx is even then)
     const bool vec = (vin.sy % 2 == 0) && ((uintptr_t)(vin.base - 1) % 8 == 0) && ((uintptr_t)(vl.base - 1) % 8 == 0);
     if (n[0] <= SL_MAXX) {
-      const size_t smem = (size_t)SL_NS * 2 * slab_stage_bytes(gx) + SL_NS * sizeof(uint64_t);
+      if (int rc = slab_prepare()) return rc;
+      const size_t smem = slab_smem_bytes(n[0]);
       auto kern = vec ? heat_step_f32_slab_kernel<true> : heat_step_f32_slab_kernel<false>;
-      NEBO_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       const int bx = (n[0] + 31) / 32 * 32, yb = (n[1] + SL_R - 1) / SL_R;
-      int bps = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, bx, smem) != cudaSuccess || bps < 1) {
-        cudaGetLastError();
-        bps = 1;
-      }
+      static std::atomic<int> per_width[2][SL_MAXX + 1];  // zero: not queried
+      const int bps = blocks_per_sm(kern, bx, per_width[vec][n[0]], smem);
       // one wave of resident blocks, chunks of 3 planes or more
       const int ch = max(1, min(num_sms() * bps / yb, (n[2] + 2) / 3));
       const int zc = (n[2] + ch - 1) / ch;
