@@ -463,8 +463,10 @@ extern "C" int nebo_reduce(const nebo_field* f, int op, int interior, double* re
         LaunchScope ls("reduce_slot", s);
         launch_slot(g, op, blocks, slot, sres, s);
       }
-      NEBO_LAUNCH_CHECK("nebo_reduce");
-      NEBO_CUDA_TRY(cudaStreamSynchronize(s));
+      // whatever the launch check says, a kernel that did start has left the slot before it is free
+      const cudaError_t launched = cudaGetLastError(), ended = cudaStreamSynchronize(s);
+      if (launched != cudaSuccess || ended != cudaSuccess)
+        return cuda_fail(launched != cudaSuccess ? launched : ended, "nebo_reduce");
       *result = *(volatile double*)hres;
       return NEBO_OK;
     };

@@ -21,6 +21,7 @@ int fail(int status, const char* fmt, ...) {
 
 int cuda_fail(cudaError_t e, const char* where) {
   if (e == cudaSuccess) return NEBO_OK;
+  cudaGetLastError();  // reported here: the next launch check must not find it again
   if (e == cudaErrorMemoryAllocation) return fail(NEBO_ERR_ALLOC, "Nebo error in %s: %s", where, cudaGetErrorString(e));
   if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver)
     return fail(NEBO_ERR_NO_DEVICE, "Nebo error in %s: %s", where, cudaGetErrorString(e));
