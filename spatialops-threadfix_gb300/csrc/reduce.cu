@@ -1,19 +1,19 @@
 // Reductions nebo_sum / nebo_max / nebo_min / nebo_norm (and _interior) over one field
 // (spatialops/NeboReductions.h:45-240).  The reference folds serially on the CPU; here a
 // deterministic tree runs on the device:
-//   per thread: batches of 8 independent loads, pairwise sums of each batch folded into a
-//               Neumaier-compensated FP64 sum (or max/min keys); a region that is one run of
-//               memory is walked as such, others a warp per row;
+//   per thread: batches of 8 independent loads, each batch summed exactly in 128-bit fixed point
+//               and folded into a Neumaier-compensated FP64 sum (or max/min keys); a region that is
+//               one run of memory is walked as such, others a warp per row;
 //   per block:  the threads' sums (and compensations) add exactly in 128-bit fixed point, max/min
 //               as order-preserving integer keys: one (sum, rest) pair or extremum per block;
 //   last step:  the blocks' pairs add the same way, rounded once.
-// What bounds it: a small field its chain of dependent steps, a large one the FP64 pipe (1.4
-// operations per element; 256^3 FP64 doubles: 40 us of it against 20 us of HBM time).  An FP64
+// What bounds it: a small field its chain of dependent steps, a large one the integer pipe (about 50
+// instructions per element of a sum beside 0.6 FP64 operations; 20 us of HBM time at 256^3).  An FP64
 // instruction holds its SM's pipe for 16 clocks a warp, so a shuffle tree of compensated adds (35
 // of them per warp) cost more than reading a 66^3 field: 23 us a field plus 11 us for the merge;
 // the integer tree takes none.  Measured, kernels of one nebo_sum: 66^3 34 -> 5 us (with nebo_reduce's
 // single launch and no device-to-host copy 60 -> 23 us per call from Python, 14.6 from C), 258^3 FP64
-// 59 us, max 35 us.
+// 63 us, max 35 us.
 // FP32 fields are accumulated in FP64.  max/min use the reference's comparisons
 // ((r < v) ? v : r and (r > v) ? v : r: NaNs never win), so they are exact; equal zeros of opposite
 // sign may come back with either sign.
@@ -177,6 +177,35 @@ __device__ __forceinline__ double sumsq8(const double* v) {
   return (a + b) + (c + d);
 }
 
+// a += the 8 values of q, with their rounding errors (every element counts as in one compensated
+// sum).  With E their largest biased exponent each becomes an integer in units of 2^(E-1141); the
+// integers add exactly and enter a as a pair: 5 FP64 operations per batch where compensated adds of
+// the elements take 5 each (250^3: 137 us of nebo_sum).  Scales whose result could leave the normal
+// range, infinities and NaNs take those.
+__device__ __forceinline__ void add8(Acc& a, const double* q) {
+  unsigned top = 0u;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) top = max(top, (unsigned)(__double_as_longlong(q[i]) >> 32) & 0x7fffffffu);
+  const int E = (int)(top >> 20);
+  if (E < 140 || E > 2020) {
+    unsigned long long any = 0ull;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) any |= (unsigned long long)__double_as_longlong(q[i]) << 1;
+    if (any) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) two_sum_add(a, q[i]);
+    }
+    return;
+  }
+  fixmath::fix128 t = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) t += fixmath::to_units(q[i], E + 3);
+  const int u = E + 3 - 1144;
+  const double s = fixmath::units_to_double0(t, u);
+  two_sum_add(a, s);
+  a.c += fixmath::units_to_double0(t - fixmath::to_units(s, E + 3), u);
+}
+
 // One thread's share of a reduction: a (sum, compensation) pair, or the extremum's key in c's place.
 template <typename T, int OP>
 __device__ __forceinline__ Acc reduce_region(const Region<T>& g) {
@@ -195,7 +224,10 @@ __device__ __forceinline__ Acc reduce_region(const Region<T>& g) {
         }
       }
     } else {
-      two_sum_add(a, OP == NEBO_RED_NORM ? sumsq8(v) : sum8(v));
+      double q[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) q[i] = OP == NEBO_RED_NORM ? v[i] * v[i] : v[i];
+      add8(a, q);
     }
   });
   if constexpr (ext) a.c = __longlong_as_double(key);
