@@ -159,10 +159,10 @@ __device__ __forceinline__ void partial_and_finish(Acc4 acc, Acc4* partials, int
   }
   a = block_reduce4(a);
   if (tid == 0) {
-    out4[0] = a.s + a.sc;
+    out4[0] = pair_sum(a.s, a.sc);
     out4[1] = a.mx == LLONG_MIN ? -INFINITY : from_key(a.mx);
     out4[2] = a.mn == LLONG_MAX ? INFINITY : from_key(a.mn);
-    out4[3] = sqrt(a.q + a.qc);
+    out4[3] = sqrt(pair_sum(a.q, a.qc));
   }
 }
 

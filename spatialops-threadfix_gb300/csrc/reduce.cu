@@ -52,8 +52,8 @@ __device__ __forceinline__ void two_sum_add(Acc& a, double v) {
 // thread 0 of the block (RED_THREADS threads).  With E the largest biased exponent of all of them,
 // each becomes an integer in units of 2^(E-1134) (|x| < 2^112; anything down to 2^-59 of the
 // largest keeps its 53 bits, the rest is within 2^-113 of it) and the 512 integers add exactly.
-// Infinities and NaNs give NaN, as the compensation does; scales whose result could leave the
-// normal range add in FP64.
+// Infinities of one sign give that infinity, others and NaNs NaN (s decides: a compensation beside an
+// infinite s is NaN); scales whose result could leave the normal range add in FP64.
 __device__ __forceinline__ Acc block_sum(Acc a) {
   __shared__ int she[RED_THREADS / 32];
   __shared__ fixmath::fix128 shs[RED_THREADS / 32];
@@ -65,10 +65,17 @@ __device__ __forceinline__ Acc block_sum(Acc a) {
 #pragma unroll
   for (int i = 0; i < RED_THREADS / 32; ++i) E = max(E, she[i]);
   if (E < 140 || E > 2020) {  // block-uniform
-    if (E == 0x7ff || !__syncthreads_or(((unsigned long long)__double_as_longlong(a.s) << 1) != 0 ||
-                                        ((unsigned long long)__double_as_longlong(a.c) << 1) != 0)) {
-      a.s = E == 0x7ff ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
+    if (E == 0x7ff) {
+      const long long PINF = 0x7ff0000000000000LL, b = __double_as_longlong(a.s);
+      const bool nan = (b & ~(1LL << 63)) > PINF;
+      const bool pos = __syncthreads_or(nan || b == PINF), neg = __syncthreads_or(nan || b == (PINF | (1LL << 63)));
+      a.s = __longlong_as_double(pos == neg ? 0x7ff8000000000000LL : (pos ? PINF : PINF | (1LL << 63)));
       a.c = 0.0;
+      return a;
+    }
+    if (!__syncthreads_or(((unsigned long long)__double_as_longlong(a.s) << 1) != 0 ||
+                          ((unsigned long long)__double_as_longlong(a.c) << 1) != 0)) {
+      a.s = a.c = 0.0;
       return a;
     }
     __shared__ Acc sha[RED_THREADS];
@@ -80,6 +87,7 @@ __device__ __forceinline__ Acc block_sum(Acc a) {
         two_sum_add(r, sha[i].s);
         r.c += sha[i].c;
       }
+      if (fixmath::dexp(r.s) == 0x7ff) r.c = 0.0;
       a = r;
     }
     return a;
@@ -629,10 +637,10 @@ __global__ void __launch_bounds__(RED_THREADS, 4) reduce4_final_kernel(const Acc
   for (int i = threadIdx.x; i < n; i += RED_THREADS) merge4(a, partials[i]);
   a = block_acc4(a);
   if (threadIdx.x == 0) {
-    out[0] = a.s + a.sc;
+    out[0] = pair_sum(a.s, a.sc);
     out[1] = a.mx == LLONG_MIN ? -INFINITY : from_key(a.mx);
     out[2] = a.mn == LLONG_MAX ? INFINITY : from_key(a.mn);
-    out[3] = sqrt(a.q + a.qc);
+    out[3] = sqrt(pair_sum(a.q, a.qc));
   }
 }
 

@@ -22,6 +22,8 @@ struct Acc4 {
 __device__ __forceinline__ double from_key(long long k) {
   return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
 }
+// A sum and its compensation (NaN beside an infinite sum).
+__device__ __forceinline__ double pair_sum(double s, double c) { return isinf(s) ? s : s + c; }
 __device__ __forceinline__ void comp_add(double& s, double& c, double v) {
   const double t = s + v;
   c += (fabs(s) >= fabs(v)) ? ((s - t) + v) : ((v - t) + s);
