@@ -19,10 +19,13 @@
 // spacing evaluates the reference's own form (same operations, same order).  Both use _rn
 // intrinsics so no multiply-add is contracted.  FP32 (storage and arithmetic) uses the scaled
 // form with per-direction weights (its operations: face_f32 and what follows it).
+#include <atomic>
 #include <climits>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <tuple>
+#include <vector>
 
 #include "common.cuh"
 #include "fp64_int.cuh"
@@ -1484,38 +1487,141 @@ struct GraphKey {
                     o.sp[1], o.sp[2]);
   }
 };
-std::mutex g_graph_mu;
-std::map<GraphKey, cudaGraphExec_t> g_graphs;
-
-// Launch the graph cached for key on s, capturing body(capture stream) into it the first time.
-template <class Body>
-int graph_launch(const GraphKey& key, Body body, cudaStream_t s, const char* what) {
+// A cached graph, and the scratch its kernels use (three fields for the face coefficients).  The
+// scratch lies outside the graph: allocation nodes made the first call of a short run 45 to 60 us
+// longer (capture and instantiation), and a graph keeps their memory for good.
+struct GraphEntry {
   cudaGraphExec_t exec = nullptr;
+  double* scratch = nullptr;
+  size_t bytes = 0;
+  cudaEvent_t done = nullptr;  // recorded after the scratch's allocation and after each launch
+  std::mutex launch;           // an executable graph is launched by one thread at a time
+  unsigned long long used = 0;  // g_graph_clock of the last launch
+  GraphEntry() = default;
+  GraphEntry(const GraphEntry&) = delete;
+  GraphEntry& operator=(const GraphEntry&) = delete;
+  ~GraphEntry();
+};
+constexpr size_t GRAPH_SCRATCH = 128ul << 20;  // bytes of scratch that the cached graphs hold in all
+constexpr size_t GRAPH_FIELDS = 8ul << 20;     // and one graph of them: see nebo_heat_run
+constexpr size_t GRAPH_COUNT = 1024;         // cached graphs
+// Graphs that none of the last GRAPH_IDLE launches used (of a time step that has changed, of fields
+// that are gone) are dropped when there is no room for another: those that a program goes round
+// stay, and a full cache never drops what the next calls need.
+constexpr unsigned long long GRAPH_IDLE = 512;
+std::mutex g_graph_mu;
+auto& g_graphs = *new std::map<GraphKey, std::shared_ptr<GraphEntry>>;  // (outlives the CUDA runtime's exit)
+unsigned long long g_graph_clock = 0;                                   // launches
+std::atomic<size_t> g_graph_scratch{0};
+
+GraphEntry::~GraphEntry() {
+  // (a wait for this event is no part of any capture that another thread has going)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!done || cudaEventSynchronize(done) == cudaSuccess) {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (scratch) cudaFree(scratch);
+    if (done) cudaEventDestroy(done);
+  }  // else: the context is lost, and its memory with it
+  cudaGetLastError();
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  g_graph_scratch -= bytes;
+}
+
+// Room for one more graph with `bytes` of scratch (taken from the budget on success).
+bool graph_room(size_t bytes) {
+  std::vector<std::shared_ptr<GraphEntry>> idle;  // destroyed after the lock is gone
+  std::unique_lock<std::mutex> g(g_graph_mu);
+  if (g_graphs.size() >= GRAPH_COUNT || (bytes && g_graph_scratch + bytes > GRAPH_SCRATCH)) {
+    for (auto it = g_graphs.begin(); it != g_graphs.end();) {
+      if (it->second->used + GRAPH_IDLE <= g_graph_clock) {
+        idle.push_back(std::move(it->second));
+        it = g_graphs.erase(it);
+      } else {
+        ++it;
+      }
+    }
+    g.unlock();
+    idle.clear();
+    g.lock();
+  }
+  if (bytes && g_graph_scratch + bytes > GRAPH_SCRATCH) return false;
+  g_graph_scratch += bytes;
+  return true;
+}
+
+// Launch the graph cached for key on s, capturing body(capture stream, scratch) into it the first
+// time.  scratch: bytes that the body's kernels need; *fits is false, and nothing launched, where they
+// are not to be had.
+template <class Body>
+int graph_launch(const GraphKey& key, size_t scratch, Body body, cudaStream_t s, const char* what, bool* fits) {
+  *fits = true;
+  std::shared_ptr<GraphEntry> e;
+  std::unique_lock<std::mutex> turn;
   {
     std::lock_guard<std::mutex> g(g_graph_mu);
     auto it = g_graphs.find(key);
-    if (it != g_graphs.end()) exec = it->second;
+    if (it != g_graphs.end()) {
+      e = it->second;
+      e->used = ++g_graph_clock;
+    }
   }
-  if (!exec) {
+  if (!e) {
+    e = std::make_shared<GraphEntry>();
+    // no other thread launches it before this one: later launches are ordered behind the first, and so
+    // behind the scratch's allocation on s
+    turn = std::unique_lock<std::mutex>(e->launch);
+    if (!graph_room(scratch)) {
+      *fits = false;
+      return NEBO_OK;
+    }
+    e->bytes = scratch;
+    NEBO_CUDA_TRY(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
+    if (scratch) {
+      const cudaError_t err = cudaMallocAsync((void**)&e->scratch, scratch, s);
+      if (err != cudaSuccess) {
+        cudaGetLastError();
+        e->scratch = nullptr;
+        *fits = false;
+        return NEBO_OK;
+      }
+      NEBO_CUDA_TRY(cudaEventRecord(e->done, s));
+    }
     cudaStream_t cap;
     NEBO_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    NEBO_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-    const int rc = body(cap);
+    cudaError_t err = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+    if (err != cudaSuccess) {
+      cudaStreamDestroy(cap);
+      return cuda_fail(err, what);
+    }
+    const int rc = body(cap, e->scratch);
     cudaGraph_t graph = nullptr;
-    cudaError_t e = cudaStreamEndCapture(cap, &graph);
+    err = cudaStreamEndCapture(cap, &graph);
     cudaStreamDestroy(cap);
     if (rc) {
       if (graph) cudaGraphDestroy(graph);
       return rc;
     }
-    if (e != cudaSuccess) return cuda_fail(e, what);
-    e = cudaGraphInstantiate(&exec, graph, 0);
+    if (err != cudaSuccess) return cuda_fail(err, what);
+    err = cudaGraphInstantiate(&e->exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return cuda_fail(e, what);
+    if (err != cudaSuccess) {
+      e->exec = nullptr;
+      return cuda_fail(err, what);
+    }
     std::lock_guard<std::mutex> g(g_graph_mu);
-    g_graphs[key] = exec;
+    auto it = g_graphs.emplace(key, e).first;
+    if (it->second != e) {  // another thread was first
+      turn.unlock();
+      turn.release();
+      e = it->second;
+    }
+    e->used = ++g_graph_clock;
   }
-  NEBO_CUDA_TRY(cudaGraphLaunch(exec, s));
+  if (!turn.owns_lock()) turn = std::unique_lock<std::mutex>(e->launch);
+  NEBO_CUDA_TRY(cudaGraphLaunch(e->exec, s));
+  // (launched into a graph that the caller records, it is copied there)
+  if (!stream_capturing(s)) NEBO_CUDA_TRY(cudaEventRecord(e->done, s));
   return NEBO_OK;
 }
 
@@ -1610,17 +1716,10 @@ bool heat_faces_ok(const nebo_field* f) { return (long)f->glob[0] * f->glob[1] <
 namespace {
 
 // The steps of nebo_heat_run one launch at a time (T's ghosts filled): FP64 on face coefficients in
-// scratch of three fields when `soft`, else (or when the scratch does not fit) on lambda.
+// lf (scratch of three fields), or on lambda where that is null.
 int heat_run_steps(const nebo_field* T, const nebo_field* Ttmp, const nebo_field* lam, int steps, double dt,
-                   const double sp[3], bool soft, cudaStream_t s) {
+                   const double sp[3], double* lf, cudaStream_t s) {
   const size_t cells = (size_t)T->glob[0] * T->glob[1] * T->glob[2];
-  double* lf = nullptr;
-  if (soft) {
-    if (cudaMallocAsync((void**)&lf, 3 * cells * sizeof(double), s) != cudaSuccess) {
-      cudaGetLastError();
-      lf = nullptr;
-    }
-  }
   int rc = NEBO_OK;
   const double* faces[3] = {nullptr, nullptr, nullptr};
   if (lf) {
@@ -1639,7 +1738,6 @@ int heat_run_steps(const nebo_field* T, const nebo_field* Ttmp, const nebo_field
         cudaMemcpyAsync(T->data, Ttmp->data, cells * elem_size(T->dtype), cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) rc = cuda_fail(e, "nebo_heat_run copy");
   }
-  if (lf) cudaFreeAsync(lf, s);
   return rc;
 }
 
@@ -1697,7 +1795,8 @@ extern "C" int nebo_heat_run_ex(const nebo_field* T, const nebo_field* Ttmp, con
   if (!graph) return body(s);
   GraphKey key{T->data, Ttmp->data, lam->data, {T->glob[0], T->glob[1], T->glob[2]}, T->dtype, steps, mode, dt,
                {1.0, 1.0, 1.0}};
-  return graph_launch(key, body, s, what);
+  bool fits;
+  return graph_launch(key, 0, [&](cudaStream_t cap, double*) { return body(cap); }, s, what, &fits);
 }
 
 extern "C" int nebo_heat_run(const nebo_field* T, const nebo_field* Ttmp, const nebo_field* lam, int steps, double dt,
@@ -1714,21 +1813,31 @@ extern "C" int nebo_heat_run(const nebo_field* T, const nebo_field* Ttmp, const 
   // FP64 runs of a few steps compute lambda's face coefficients once: that pass costs 0.1 ms at
   // 256^3 (4 us at 64^3) and each step then saves 0.2 ms (2 us), in general spacing 0.48 ms (8 us).
   // Graphs that the caller records keep the other form: scratch would put allocation nodes into
-  // them.  Fields whose scratch would hold
-  // more than 1 GB in a cached graph are launched step by step: their steps are long enough.
+  // them.
   const size_t scratch = 3 * (size_t)T->glob[0] * T->glob[1] * T->glob[2] * sizeof(double);
   const bool soft =
       T->dtype == NEBO_F64 && steps >= (heat_unit(sp) ? 3 : 2) && heat_faces_ok(T) && !stream_capturing(s);
-  if (soft) pool_retain();  // a pool setting: not from inside the capture below
-  if (!use_graph || (soft && scratch > (1ul << 30))) return heat_run_steps(T, Ttmp, lam, steps, dt, sp, soft, s);
-  GraphKey key{T->data, Ttmp->data, lam->data, {T->glob[0], T->glob[1], T->glob[2]}, T->dtype, steps, soft ? -2 : -1,
-               dt, {sp[0], sp[1], sp[2]}};
-  auto body = [&](cudaStream_t cap) { return heat_run_steps(T, Ttmp, lam, steps, dt, sp, soft, cap); };
-  rc = graph_launch(key, body, s, "nebo_heat_run");
-  if (rc == NEBO_ERR_ALLOC && soft) {  // no room for the graph's scratch: the graph without it
-    key.mode = -1;
-    auto plain = [&](cudaStream_t cap) { return heat_run_steps(T, Ttmp, lam, steps, dt, sp, false, cap); };
-    rc = graph_launch(key, plain, s, "nebo_heat_run");
+  if (soft) pool_retain();
+  if (use_graph) {
+    GraphKey key{T->data, Ttmp->data, lam->data, {T->glob[0], T->glob[1], T->glob[2]}, T->dtype, steps, soft ? -2 : -1,
+                 dt, {sp[0], sp[1], sp[2]}};
+    auto body = [&](cudaStream_t cap, double* lf) { return heat_run_steps(T, Ttmp, lam, steps, dt, sp, lf, cap); };
+    bool fits;
+    if (!soft || scratch <= GRAPH_FIELDS) {
+      rc = graph_launch(key, soft ? scratch : 0, body, s, "nebo_heat_run", &fits);
+      if (fits) return rc;
+    }
   }
+  // Step by step, also where the cached graphs' scratch has no room for three fields more.  Fields of
+  // more than 0.35 M cells always: their steps take 15 us or more and the launch of one 2 us, so a
+  // graph gains nothing, and capturing it and mapping its scratch lengthen a first call (16 steps at
+  // 96^3: first 600 and then 414 us in a graph, 437 and 416 so; 64^3 in a graph 294 and 181).
+  double* lf = nullptr;
+  if (soft && cudaMallocAsync((void**)&lf, scratch, s) != cudaSuccess) {
+    cudaGetLastError();
+    lf = nullptr;  // every step on lambda
+  }
+  rc = heat_run_steps(T, Ttmp, lam, steps, dt, sp, lf, s);
+  if (lf) cudaFreeAsync(lf, s);
   return rc;
 }
