@@ -157,6 +157,22 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<float> a
   }
 }
 
+// The cells (x, y, z0 .. z1-1) of an FP64 stage that came out infinite or NaN, in the form that sums the
+// four weighted values and halves before it adds.  The shorter form (below) leaves the doubles earlier:
+// 27 (phi - phi) from differences of 6.6e306 on, the sum of two states above 9e307; here the operator's
+// own infinities and NaNs remain.  Rare, so apart from the march, which only notes that a value left.
+__device__ __noinline__ void restage_column_f64(const TrArgs<double>& a, int x, int y, int z0, int z1, bool second) {
+  for (int z = z0; z < z1; ++z) {
+    const long c = (long)x + (long)a.sy * y + a.sz * z;
+    if (((__double_as_longlong(a.out64[c]) >> 52) & 0x7ff) != 0x7ff) continue;
+    const double rhs = ((face_flux(a, c + 1, 1, a.u) - face_flux(a, c, 1, a.u)) +
+                        (face_flux(a, c + a.sy, a.sy, a.v) - face_flux(a, c, a.sy, a.v))) +
+                       (face_flux(a, c + a.sz, a.sz, a.w) - face_flux(a, c, a.sz, a.w));
+    const double r = a.phi[c] + a.dt * rhs;
+    store_images2(a.out64, a.sy, a.sz, x, y, z, a.n, second ? 0.5 * a.base[c] + 0.5 * r : r);
+  }
+}
+
 // FP64 stage.  Per face, with d1 = phi[f] - phi[f-s] and d3 = phi[f+s] - phi[f-2s],
 //   F = k (27 d1 - d3) - u up,   k = nu (lambda[f-s] + lambda[f]) / 48:
 // 5 FP64 operations (two more where k is not precomputed), the upwind value picked by u's bits; the
@@ -166,7 +182,7 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<float> a
 // the four weighted values and compares u in FP64), 79 % busy: 188 -> 110 us per stage at 127^3.
 // Error against 80-bit arithmetic after 20 steps: 1.15e-16 (2-norm), as before (1.16e-16).
 template <bool SECOND, bool KF>
-__global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<double> a,
+__global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(const __grid_constant__ TrArgs<double> a,
                                                                         const double* __restrict__ kfx,
                                                                         const double* __restrict__ kfy,
                                                                         const double* __restrict__ kfz, double kc,
@@ -201,6 +217,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
   long c = c0 + sz * z0;
   double pm1 = ld_step(a.phi + c - sz), p0 = ld_step(a.phi + c), p1 = ld_step(a.phi + c + sz);
   double fzlo = flux(coef(kfz, c, sz), ld_step(a.w + c), ld_step(a.phi + c - 2 * sz), pm1, p0, p1);
+  bool left = false;  // a value of this column left the doubles
 #pragma unroll 1
   for (int z = z0; z < z1; ++z, c += sz) {
     const int buf = z & 1;
@@ -253,6 +270,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
         const int e = (int)((b >> 52) & 0x7ff);
         r = e >= 2 && e < 0x7ff ? __longlong_as_double(b - (1LL << 52)) : 0.5 * r;
       }
+      left = left || ((__double_as_longlong(r) >> 52) & 0x7ff) == 0x7ff;
       store_images2(a.out64, sy, sz, x, y, z, n, r);
     }
     fzlo = fzhi;
@@ -260,6 +278,7 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<d
     p0 = p1;
     p1 = p2;
   }
+  if (left) restage_column_f64(a, x, y, z0, z1, SECOND);
 }
 
 // k of every face of the stages above (cells 0 .. n of each axis: n is the high face of the last
@@ -853,6 +872,12 @@ extern "C" int nebo_transport_run(double* phi, const void* u, const void* v, con
     a.sy = (int)sy;
     a.sz = sz;
     a.dt = dt;
+    a.nu = nu;
+    const double h = 1.0 / 24.0;
+    a.q0 = h;
+    a.q1 = -27.0 * h;
+    a.q2 = 27.0 * h;
+    a.q3 = -h;
     const double kc = nu / 48.0;
     // The face coefficients once per run, in scratch of three fields, where they pay (their pass
     // costs about a fifth of a stage and saves an eighth of each) and the caller records no graph;
