@@ -150,8 +150,8 @@ int nebo_heat_step(const nebo_field* T, const nebo_field* Tout, const nebo_field
  * in scratch of three fields from the stream-ordered pool (given back to it at the end of the run;
  * cached graphs keep theirs, 128 MiB in all, and fields above 0.35 M cells, for which a graph gains
  * nothing, are launched step by step instead).  Where that memory is not to be had, and while the
- * caller records a graph, every step forms them.  The bits are the same.  At most 1024 graphs are
- * cached; those that the last 512 graph runs did not use make room for others. */
+ * caller records a graph, every step forms them.  The bits are the same.  About 1024 graphs
+ * are cached; those that the last 512 graph runs did not use make room for others. */
 int nebo_heat_run(const nebo_field* T, const nebo_field* Ttmp, const nebo_field* lam, int steps,
                   double dt, const double spacing[3], int use_graph, nebo_stream_t stream);
 

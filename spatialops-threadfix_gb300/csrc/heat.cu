@@ -1494,9 +1494,9 @@ struct GraphEntry {
   cudaGraphExec_t exec = nullptr;
   double* scratch = nullptr;
   size_t bytes = 0;
-  cudaEvent_t done = nullptr;  // recorded after the scratch's allocation and after each launch
+  cudaEvent_t done = nullptr;  // of the scratch: recorded after its allocation and after each launch
   std::mutex launch;           // an executable graph is launched by one thread at a time
-  unsigned long long used = 0;  // g_graph_clock of the last launch
+  unsigned long long used = 0;  // g_graph_clock of the last run
   GraphEntry() = default;
   GraphEntry(const GraphEntry&) = delete;
   GraphEntry& operator=(const GraphEntry&) = delete;
@@ -1504,14 +1504,15 @@ struct GraphEntry {
 };
 constexpr size_t GRAPH_SCRATCH = 128ul << 20;  // bytes of scratch that the cached graphs hold in all
 constexpr size_t GRAPH_FIELDS = 8ul << 20;     // and one graph of them: see nebo_heat_run
-constexpr size_t GRAPH_COUNT = 1024;         // cached graphs
-// Graphs that none of the last GRAPH_IDLE launches used (of a time step that has changed, of fields
+constexpr size_t GRAPH_COUNT = 1024;           // cached graphs
+// Graphs that none of the last GRAPH_IDLE runs used (of a time step that has changed, of fields
 // that are gone) are dropped when there is no room for another: those that a program goes round
 // stay, and a full cache never drops what the next calls need.
 constexpr unsigned long long GRAPH_IDLE = 512;
 std::mutex g_graph_mu;
 auto& g_graphs = *new std::map<GraphKey, std::shared_ptr<GraphEntry>>;  // (outlives the CUDA runtime's exit)
-unsigned long long g_graph_clock = 0;                                   // launches
+unsigned long long g_graph_clock = 0;                                   // runs that asked for a graph
+unsigned long long g_graph_scan = 0;  // the run from which idle graphs are looked for again
 std::atomic<size_t> g_graph_scratch{0};
 
 GraphEntry::~GraphEntry() {
@@ -1532,7 +1533,9 @@ GraphEntry::~GraphEntry() {
 bool graph_room(size_t bytes) {
   std::vector<std::shared_ptr<GraphEntry>> idle;  // destroyed after the lock is gone
   std::unique_lock<std::mutex> g(g_graph_mu);
-  if (g_graphs.size() >= GRAPH_COUNT || (bytes && g_graph_scratch + bytes > GRAPH_SCRATCH)) {
+  if (g_graph_clock >= g_graph_scan &&
+      (g_graphs.size() >= GRAPH_COUNT || (bytes && g_graph_scratch + bytes > GRAPH_SCRATCH))) {
+    g_graph_scan = g_graph_clock + 32;  // not on every call of a full cache
     for (auto it = g_graphs.begin(); it != g_graphs.end();) {
       if (it->second->used + GRAPH_IDLE <= g_graph_clock) {
         idle.push_back(std::move(it->second));
@@ -1560,10 +1563,11 @@ int graph_launch(const GraphKey& key, size_t scratch, Body body, cudaStream_t s,
   std::unique_lock<std::mutex> turn;
   {
     std::lock_guard<std::mutex> g(g_graph_mu);
+    ++g_graph_clock;
     auto it = g_graphs.find(key);
     if (it != g_graphs.end()) {
       e = it->second;
-      e->used = ++g_graph_clock;
+      e->used = g_graph_clock;
     }
   }
   if (!e) {
@@ -1576,8 +1580,8 @@ int graph_launch(const GraphKey& key, size_t scratch, Body body, cudaStream_t s,
       return NEBO_OK;
     }
     e->bytes = scratch;
-    NEBO_CUDA_TRY(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
     if (scratch) {
+      NEBO_CUDA_TRY(cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming));
       const cudaError_t err = cudaMallocAsync((void**)&e->scratch, scratch, s);
       if (err != cudaSuccess) {
         cudaGetLastError();
@@ -1616,12 +1620,11 @@ int graph_launch(const GraphKey& key, size_t scratch, Body body, cudaStream_t s,
       turn.release();
       e = it->second;
     }
-    e->used = ++g_graph_clock;
+    e->used = g_graph_clock;
   }
   if (!turn.owns_lock()) turn = std::unique_lock<std::mutex>(e->launch);
   NEBO_CUDA_TRY(cudaGraphLaunch(e->exec, s));
-  // (launched into a graph that the caller records, it is copied there)
-  if (!stream_capturing(s)) NEBO_CUDA_TRY(cudaEventRecord(e->done, s));
+  if (e->scratch) NEBO_CUDA_TRY(cudaEventRecord(e->done, s));
   return NEBO_OK;
 }
 
