@@ -126,14 +126,15 @@ __host__ __device__ __forceinline__ int fbits(float x) {
 }
 __host__ __device__ __forceinline__ uint64_t uabs(int64_t a) { return a < 0 ? 0 - (uint64_t)a : (uint64_t)a; }
 
-// A double at 2^S modulo 2^64, truncated toward zero (|v| 2^S < 2^64; 0 for subnormals).
+// A double at 2^S modulo 2^64, truncated toward zero (|v| 2^S < 2^64).  Zeros and subnormals, whose
+// implicit bit is not masked off, give +-1: one unit of 2^-S, far below a caller's last bit.
 template <int S>
 __host__ __device__ __forceinline__ int64_t to_fix_small(double v) {
   const uint64_t b = bits(v);
   const int e = (int)((b >> 52) & 0x7ff);
   const uint64_t m = ((b & 0xfffffffffffffULL) | 0x10000000000000ULL) << 11;  // v = m 2^(e - 1086)
   const int sh = 1086 - S - e;
-  const uint64_t f = m >> (sh < 63 ? sh : 63);  // (a zero's m has its top bit alone above the shift)
+  const uint64_t f = m >> (sh < 63 ? sh : 63);  // (at most the top bit remains: a zero's unit)
   return (int64_t)b < 0 ? -(int64_t)f : (int64_t)f;
 }
 

@@ -120,10 +120,12 @@ inline bool stream_capturing(cudaStream_t s) {
 // Launch of a step kernel that follows its like in a stream (programmatic dependent launch).  Its
 // blocks may be launched once every block of the kernel before has called step_end or ended; they
 // wait in step_begin, before they touch memory, until that kernel has finished and its writes are
-// visible.  Every kernel launched so calls step_begin first and step_end when a block has only its
-// last plane to store: called at the start, the next kernel's blocks take the free slots of some SMs
-// early and its own work is then unevenly spread (64^3 heat steps 10.1 -> 16.8 us; at the end 9.7,
-// and 12.5 -> 10.0 for launches outside a graph).
+// visible.  Every kernel launched so calls step_begin first and step_end, if at all, late: at a
+// block's last plane (the patch kernels, whose blocks take several items, after the last one; the
+// FP32 slab kernel, whose 40 registers have no room for it, leaves it to its blocks' end).  Called at
+// the start, the next kernel's blocks take the free slots of some SMs early and its own work is then
+// unevenly spread (64^3 heat steps 10.1 -> 16.8 us; at the end 9.7, and 12.5 -> 10.0 for launches
+// outside a graph).
 template <class... Params, class... Args>
 inline void launch_step_kernel(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                Args... args) {

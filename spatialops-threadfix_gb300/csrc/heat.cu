@@ -1186,10 +1186,10 @@ __global__ void __launch_bounds__(BP_THREADS, 3) heat_step_f32_bulk2_kernel(cons
 // which drops cells of plane nz's ghost corner that no face reads), and the cells are read
 // (address mod 16) bytes into the stage.  Planes below 0 are not staged (the low z faces of a
 // chunk's first plane read them from global memory), so no copy starts before the field.
-// What bounds it: issue (82 instructions per cell, 59 % of the slots) and the barrier per plane;
-// 40 registers let four blocks of 352 threads share an SM (64 registers, two blocks: 42.4 us).
-// At 323 x 197 x 150: 36.9 us = 3.1 TB/s, where 4-byte cp.async copies per cell took 108 us;
-// 322 x 198 x 150 (8-byte copies before) 69.8 -> 36.9, 401 x 301 x 201 141 -> 82.
+// What bounds it: issue (92 instructions per cell, 94 at even pitches, 69 % of the slots) and the
+// barrier per plane; 40 registers let four blocks of 352 threads share an SM (64 registers, two
+// blocks, took 15 % longer).  At 323 x 197 x 150: 34.9 us = 3.3 TB/s, where 4-byte cp.async copies
+// per cell took 108 us; 322 x 198 x 150 (8-byte copies before) 69.8 -> 35.0, 401 x 301 x 201 141 -> 82.
 constexpr int SL_R = 4;        // rows per block (the scalar arithmetic's row period)
 constexpr int SL_NS = 3;       // stages
 constexpr int SL_MAXX = 1024;  // threads per block
@@ -1379,7 +1379,8 @@ int launch_heat(const nebo_field* Tf, const nebo_field* Tof, const nebo_field* L
   } else {
     // bulk-copied slabs in packed pairs: rows of 16-byte aligned windows with an even pitch, 8 rows
     // per block.  Its 128 pair columns want wide rows: against the scalar slab kernel below it takes
-    // 45.3 : 56.6 us at 256 columns, 37.0 : 41.1 at 224, 46.4 : 44.7 at 192, 34.9 : 24.6 at 64.
+    // 44.3 : 55.5 us at 256 columns (x 256 x 256), 44.2 : 49.5 at 224, 44.1 : 49.6 at 208, 45.3 : 43.2
+    // at 192, 36.4 : 31.4 at 128, 32.9 : 24.0 at 64.
     const int gx = Tf->glob[0], gy = Tf->glob[1];
     const size_t bk_smem = (size_t)BK_NS * 2 * BK_ROWS * gx * sizeof(float) + BK_NS * sizeof(uint64_t);
     const bool bulk = n[0] > 192 && n[0] <= 2 * BP_PAIRS && n[1] % BK_RY == 0 && gx % 2 == 0 && gy % 2 == 0 &&

@@ -200,9 +200,9 @@ __device__ __forceinline__ long win_flat(const PGeom& g, int i, int j, int k) {
 // particle, over its lanes 32 at a time, so every lane does the same work per pair whatever the
 // box sizes.  For CellToParticle the owner lane then adds its pairs' products in that order.
 constexpr int PB = 4;
+constexpr int PWARPS = 8;  // warps per block
 constexpr int PCAP = 512;  // CellToParticle: products held per warp before the owners add them
 enum { PM_C2P = 0, PM_FILL = 2 };
-constexpr int PWARPS = 8;  // warps per block
 
 template <int MODE>
 struct WarpShared {
@@ -253,7 +253,7 @@ __device__ __forceinline__ double serial_particle(const PGeom& g, const double* 
 // tab: the block's shared memory holds the faces of every window cell of each axis (3 FP64
 // operations per cell once, instead of once per particle and cell of its box; the window's edges
 // add up to PTAB cells or fewer).  The FP64 pipe bounds both modes (82 % busy in the gather): 2 M
-// particles, 18.8 M pairs: gather 731 -> 566 us, fill 617 -> 430 (506 with two blocks per SM; the
+// particles, 18.8 M pairs: gather 731 -> 561 us, fill 617 -> 404 (506 with two blocks per SM; the
 // gather's products leave room for two).
 constexpr int PTAB = 1024;
 
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(PWARPS * 32, MODE == PM_C2P ? 2 : 3) particles
   extern __shared__ __align__(16) unsigned char particle_smem[];
   WarpShared<MODE>* smem = reinterpret_cast<WarpShared<MODE>*>(particle_smem);
   CellFaces* faces = reinterpret_cast<CellFaces*>(particle_smem + faces_offset<MODE>());
-    if (tab) {
+  if (tab) {
     const int n0 = g.nmax[0], n1 = n0 + g.nmax[1], n2 = n1 + g.nmax[2];
     for (int i = threadIdx.x; i < n2; i += PWARPS * 32)
       faces[i] = i < n0 ? cell_faces(g, 0, i) : (i < n1 ? cell_faces(g, 1, i - n0) : cell_faces(g, 2, i - n1));

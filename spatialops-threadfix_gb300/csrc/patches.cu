@@ -385,9 +385,9 @@ constexpr int PNS = 5;
 
 // Every ghost cell of every patch of an arena takes its periodic source's value (blocks of one
 // blockIdx.y share a patch, threads over the six ghost faces: z faces whole, then y faces for the
-// interior z, then x faces for the interior y and z).  FP64 arenas after loading (one launch for
-// all patches: 512 of them took 1.9 ms a launch each); FP32 windows after a run, as the strip kernel
-// writes no ghosts during the steps.
+// interior z, then x faces for the interior y and z).  FP64 arenas after loading (512 patches, a launch
+// each, took 1.9 ms in all); FP32 windows after a run, as the strip kernel writes no ghosts during the
+// steps.
 template <typename T>
 __global__ void __launch_bounds__(256) patches_ghosts_kernel(const PatchDev* __restrict__ patches, int npatch,
                                                              T* __restrict__ arena) {
@@ -569,7 +569,8 @@ __global__ void __launch_bounds__(PT_THREADS, 2) patches_f32_strip_kernel(const 
 // neighbour of each cell by itself, 54 instructions a cell, and was bound by issue (81 %); 512
 // patches of 16..96 cells an edge (742 MB a step) took 170 us a step that way and take 122 us so
 // (6.1 TB/s; bound by memory; 131 us with three stages, 124 with five, 138 with seven, 134 at eight
-// blocks an SM, whose 32 registers spill).  The operations of a cell are those of patches_f32_strip_kernel in the same order.
+// blocks an SM, whose 32 registers spill).  The operations of a cell are those of
+// patches_f32_strip_kernel in the same order.
 // No ghost cells exist in this layout: nebo_patchset_sync writes whole FP64 windows.
 constexpr int PB_CELLS = 4 * PT_THREADS;  // floats per strip plane, the rows' padding included
 constexpr int PB_NS = 4;                  // stages
@@ -684,12 +685,13 @@ __global__ void __launch_bounds__(PT_THREADS) patches_f32_bulk_kernel(const Patc
 }
 
 // FP64 windows -> FP32 slab layout (interiors only) and back (whole windows: each cell of a
-// window takes its periodic interior source, so the ghosts are filled in the same pass).  Packing, a warp takes a row, four of its cells per lane in flight.  Unpacking, a thread
-// takes four consecutive window elements whatever rows they fall in: windows start on 256-byte
-// boundaries, so the results are two 16-byte stores on a whole sector.  Values widen and round by
-// their bits (a hardware conversion issues on the FP64 pipe).  512 patches of 16..96 cells an edge
-// back to windows (1.2 GB): an index division per cell 623 us, a warp per row with 8-byte stores 358,
-// two elements a thread 348, four 287 (4.2 TB/s).
+// window takes its periodic interior source, so the ghosts are filled in the same pass).  Packing, a
+// warp takes a row, four of its cells per lane in flight.  Unpacking, a thread takes four consecutive
+// window elements whatever rows they fall in: windows start on 256-byte boundaries, so the results are
+// two 16-byte stores on a whole sector.  Values widen and round by their bits (a hardware conversion
+// issues on the FP64 pipe).  512 patches of 16..96 cells an edge back to windows (1.2 GB): an index
+// division per cell 623 us, a warp per row with 8-byte stores 358, two elements a thread 348, four 287
+// (4.2 TB/s).
 __device__ __forceinline__ float narrow(double v) {  // rounded to nearest, subnormal floats included
   const int e = fixmath::dexp(v);
   return e <= 896 && e >= 872 ? (float)v : fixmath::f64_to_f32_rn(v);

@@ -157,32 +157,19 @@ __global__ void __launch_bounds__(TX* TY) transport_stage_kernel(TrArgs<float> a
   }
 }
 
-// The cells (x, y, z0 .. z1-1) of an FP64 stage that came out infinite or NaN, in the form that sums the
-// four weighted values and halves before it adds.  The shorter form (below) leaves the doubles earlier:
-// 27 (phi - phi) from differences of 6.6e306 on, the sum of two states above 9e307; here the operator's
-// own infinities and NaNs remain.  Rare, so apart from the march, which only notes that a value left.
-__device__ __noinline__ void restage_column_f64(const TrArgs<double>& a, int x, int y, int z0, int z1, bool second) {
-  for (int z = z0; z < z1; ++z) {
-    const long c = (long)x + (long)a.sy * y + a.sz * z;
-    if (((__double_as_longlong(a.out64[c]) >> 52) & 0x7ff) != 0x7ff) continue;
-    const double rhs = ((face_flux(a, c + 1, 1, a.u) - face_flux(a, c, 1, a.u)) +
-                        (face_flux(a, c + a.sy, a.sy, a.v) - face_flux(a, c, a.sy, a.v))) +
-                       (face_flux(a, c + a.sz, a.sz, a.w) - face_flux(a, c, a.sz, a.w));
-    const double r = a.phi[c] + a.dt * rhs;
-    store_images2(a.out64, a.sy, a.sz, x, y, z, a.n, second ? 0.5 * a.base[c] + 0.5 * r : r);
-  }
-}
-
 // FP64 stage.  Per face, with d1 = phi[f] - phi[f-s] and d3 = phi[f+s] - phi[f-2s],
-//   F = k (27 d1 - d3) - u up,   k = nu (lambda[f-s] + lambda[f]) / 48:
+//   F = k (d1 - d3 / 27) - u up,   k = (9/16) nu (lambda[f-s] + lambda[f]):
 // 5 FP64 operations (two more where k is not precomputed), the upwind value picked by u's bits; the
 // low x and y faces come from each thread and the high ones through shared memory, the z face and
-// the column's phi window (z - 1 .. z + 2) stay in registers.  The halving of the second stage is an
-// exponent step.  What bounds it: the FP64 pipe at 23 operations per cell (40 in the form that sums
-// the four weighted values and compares u in FP64), 79 % busy: 188 -> 110 us per stage at 127^3.
-// Error against 80-bit arithmetic after 20 steps: 1.15e-16 (2-norm), as before (1.16e-16).
+// the column's phi window (z - 1 .. z + 2) stay in registers.  The second stage halves its sum by an
+// exponent step, or, where the sum leaves the normal range, both terms before it adds them; d1 is not
+// scaled up: states up to the largest double stay finite where the weighted values do.
+// What bounds it: the FP64 pipe at 23 operations per cell (40 in the form that sums the four weighted
+// values and compares u in FP64): 188 -> 105 us per stage at 127^3; 5.78 ms at 512^3, of which the
+// operations take 5.3 at 595 G/s.  Its error against extended precision is that of the weighted form
+// (tests/test_gpu_transport_range.py).
 template <bool SECOND, bool KF>
-__global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(const __grid_constant__ TrArgs<double> a,
+__global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(TrArgs<double> a,
                                                                         const double* __restrict__ kfx,
                                                                         const double* __restrict__ kfy,
                                                                         const double* __restrict__ kfz, double kc,
@@ -198,11 +185,18 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(const __
   const bool active = x < n && y < n;
   const int xc = min(x, n), yc = min(y, n);  // column/row n is a ghost: valid memory
   auto positive = [](double u) { return __double_as_longlong(u) > 0; };
+  auto half = [](double v) {  // in integers: a multiplication the compiler would issue for every cell
+    const long long b = __double_as_longlong(v);
+    const long long m = b & 0x7fffffffffffffffLL;
+    const int e = (int)(m >> 52);
+    const long long h = e >= 2 ? m - (e == 0x7ff ? 0LL : 1LL << 52) : (m + ((m >> 1) & 1)) >> 1;
+    return __longlong_as_double(h | (b & (1LL << 63)));
+  };
   auto coef = [&](const double* kf, long f, long s) {
     return KF ? ld_step(kf + f) : kc * (ld_step(a.lam + f - s) + ld_step(a.lam + f));
   };
   auto flux = [&](double k, double u, double pm2, double pm1, double p0, double pp1) {
-    const double g = fma(27.0, p0 - pm1, pm2 - pp1);
+    const double g = fma(1.0 / 27.0, pm2 - pp1, p0 - pm1);
     return fma(-u, positive(u) ? pm1 : p0, k * g);
   };
   auto flux_at = [&](const double* kf, const double* vel, long f, long s) {
@@ -217,7 +211,6 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(const __
   long c = c0 + sz * z0;
   double pm1 = ld_step(a.phi + c - sz), p0 = ld_step(a.phi + c), p1 = ld_step(a.phi + c + sz);
   double fzlo = flux(coef(kfz, c, sz), ld_step(a.w + c), ld_step(a.phi + c - 2 * sz), pm1, p0, p1);
-  bool left = false;  // a value of this column left the doubles
 #pragma unroll 1
   for (int z = z0; z < z1; ++z, c += sz) {
     const int buf = z & 1;
@@ -263,14 +256,17 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(const __
     if (z + 1 == z1) step_end();
     if (active) {
       const double rhs = ((sfx[buf][ty][tx + 1] - fx) + (sfy[buf][ty + 1][tx] - fy)) + dz;
-      double r = fma(a.dt, rhs, p0);  // FP64 stages advance from the state they read
+      // FP64 stages advance from the state they read
+      double r = fma(a.dt, rhs, p0);
       if (SECOND) {
-        r = base + r;
-        const long long b = __double_as_longlong(r);
+        const double t = base + r;
+        const long long b = __double_as_longlong(t);
         const int e = (int)((b >> 52) & 0x7ff);
-        r = e >= 2 && e < 0x7ff ? __longlong_as_double(b - (1LL << 52)) : 0.5 * r;
+        if (e >= 2 && e < 0x7ff)
+          r = __longlong_as_double(b - (1LL << 52));
+        else
+          r = half(base) + fma(0.5 * a.dt, rhs, half(p0));
       }
-      left = left || ((__double_as_longlong(r) >> 52) & 0x7ff) == 0x7ff;
       store_images2(a.out64, sy, sz, x, y, z, n, r);
     }
     fzlo = fzhi;
@@ -278,7 +274,6 @@ __global__ void __launch_bounds__(TX* TY, 3) transport_stage_f64_kernel(const __
     p0 = p1;
     p1 = p2;
   }
-  if (left) restage_column_f64(a, x, y, z0, z1, SECOND);
 }
 
 // k of every face of the stages above (cells 0 .. n of each axis: n is the high face of the last
@@ -872,13 +867,7 @@ extern "C" int nebo_transport_run(double* phi, const void* u, const void* v, con
     a.sy = (int)sy;
     a.sz = sz;
     a.dt = dt;
-    a.nu = nu;
-    const double h = 1.0 / 24.0;
-    a.q0 = h;
-    a.q1 = -27.0 * h;
-    a.q2 = 27.0 * h;
-    a.q3 = -h;
-    const double kc = nu / 48.0;
+    const double kc = nu * 0.5625;
     // The face coefficients once per run, in scratch of three fields, where they pay (their pass
     // costs about a fifth of a stage and saves an eighth of each) and the caller records no graph;
     // without them every stage forms them.
