@@ -107,7 +107,8 @@ int nebo_mask_from_points(uint32_t* words, const int32_t glob[3], const int32_t 
  * nebo_sum / nebo_max / nebo_min / nebo_norm and their _interior forms
  * (spatialops/NeboReductions.h:45-240) over one field: ghost-inclusive (valid ghosts) unless
  * interior != 0.  Accumulation is FP64 for both dtypes; sums use compensated (Neumaier)
- * partials.  nebo_reduce writes *result on the host and synchronises the stream (the reference
+ * partials, and a sum that leaves the doubles, or meets infinities of one sign, is infinite.
+ * nebo_reduce writes *result on the host and synchronises the stream (the reference
  * returns the value synchronously); nebo_reduce_async leaves it in device memory. */
 int nebo_reduce(const nebo_field* f, int op, int interior, double* result, nebo_stream_t stream);
 int nebo_reduce_async(const nebo_field* f, int op, int interior, double* d_result,
@@ -140,7 +141,9 @@ int nebo_reduce_noalloc(const nebo_field* f, int op, int interior, double* d_res
  * the same pass, Tout's ghost cells as periodic images (the next step's ghost fill).
  * T, Tout, lam: SVol, one ghost layer, same shape and dtype.  spacing = {dx,dy,dz}.
  * FP64: same operations and roundings as the reference's serial walk (bit-exact).
- * FP32: FP32 storage and arithmetic. */
+ * FP32: FP32 storage and arithmetic.  The last bits depend on the window: with an even row pitch and
+ * 8-byte aligned rows of T and lam every flux is rounded before its difference is taken; others take
+ * the high x flux, and in every fourth row the low y flux, unrounded. */
 int nebo_heat_step(const nebo_field* T, const nebo_field* Tout, const nebo_field* lam, double dt,
                    const double spacing[3], nebo_stream_t stream);
 

@@ -234,7 +234,7 @@ __device__ __forceinline__ Acc reduce_region(const Region<T>& g) {
     } else {
       double q[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) q[i] = OP == NEBO_RED_NORM ? v[i] * v[i] : v[i];
+      for (int i = 0; i < 8; ++i) q[i] = OP == NEBO_RED_NORM ? __dmul_rn(v[i], v[i]) : v[i];
       add8(a, q);
     }
   });
